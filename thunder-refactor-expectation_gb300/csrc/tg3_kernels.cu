@@ -1103,101 +1103,191 @@ __global__ void k_x0(const float2* __restrict__ dat, const float* __restrict__ s
 
 // ------------------------------------------------------------------------
 // Batched FP32 "NT" GEMM on the CUDA cores: C[b][i][j] = alpha sum_k
-// A[b][i][k] B[b][j][k] (+ nrm[b][i]).  128 x 128 x 16 tiles, 256 threads,
-// 8 x 8 outputs per thread, register-staged double buffering.  Kd must be a
-// multiple of 16 and lda/ldb multiples of 4 (rows zero-padded).
-constexpr int GB_M = 128, GB_N = 128, GB_K = 16, GB_PAD = 4;
+// A[b][i][k] B[b][j][k] (+ nrm[b][i]).  128 threads as 8 x 16, TM x TN
+// outputs a thread (tile 8 TM x 16 TN), K in tiles of BK through two shared
+// buffers.  Every output is one chain of fused multiply-adds over ascending
+// k, whatever the tile.  Kd must be a multiple of BK and lda/ldb multiples of 4
+// (rows zero-padded).
+//
+// Bound by the FP32 pipe: the products go in pairs of rows (fma.rn.f32x2,
+// one issue for two multiply-adds), which leaves issue slots for the shared
+// loads.  The column operand of a pair is one value twice, a register move.
+// A shared load costs a cycle for every 128 bytes that it returns, so a warp
+// spends TM + TN cycles of the shared port on TM TN / 4 cycles of the FP32
+// pipes: 16 x 8 outputs a thread keep that at three quarters, 8 x 8 at one.
+// Measured against 128 x 128 tiles of 256 threads with single multiply-adds:
+// 6,912 x 16,317 x 768 in 2.8 instead of 4.2 ms (62 TFLOP/s, cuBLAS SGEMM 70),
+// 32 particles of 1,000 x 100 x 19,904 in 3.0 instead of 4.7 ms, one of
+// 100 x 9 x 768 in 8 instead of 13 us.
+// The staged tiles are transposed, [k][row], with row XOR f(k): f spreads the
+// BK / 4 float4 columns that a warp stores together over the banks (no
+// conflict at any BK) and moves whole float4 groups, so the reads stay vectors.
+__device__ __forceinline__ uint64_t pack2(float x, float y)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
 
-__global__ void __launch_bounds__(256, 1)
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+template <int TM, int TN>
+__global__ void __launch_bounds__(128, TM == 16 ? 2 : TM == 8 ? 3 : 4)
 k_gemm_nt_fp32(const float* __restrict__ A, long long sA, int lda,
                const float* __restrict__ B, long long sB, int ldb,
                int M, int N, int Kd, float* __restrict__ C, long long sC, int ldc,
                const float* __restrict__ nrm, long long sN, float alpha, int cGroup,
                long long cGroupStride)
 {
-    __shared__ __align__(16) float As[2][GB_K][GB_M + GB_PAD];
-    __shared__ __align__(16) float Bs[2][GB_K][GB_N + GB_PAD];
+    constexpr int BM = 8 * TM, BN = 16 * TN;
+    constexpr int BK = TM == 2 ? 32 : 128 / TM;   // 8, 16, 32, 32
+    constexpr int NA = BM * BK / 512;             // A float4 a thread and tile
+    // K tiles in flight from global memory (registers allowing)
+    constexpr int D = TM >= 8 || TN <= 4 ? 2 : 1;
+    constexpr int QK = BK / 4;                    // float4 columns of a tile
+    constexpr int PB = (BN + 31) / 32 * 32;       // column pitch of the staged B
+    constexpr int NB = (BN * QK + 127) / 128;     // B float4 a thread and tile
+    __shared__ __align__(16) float As[2][BK][(BM + 31) / 32 * 32];
+    __shared__ __align__(16) float Bs[2][BK][PB];
     const int b = blockIdx.z;
-    const int i0 = blockIdx.y * GB_M, j0 = blockIdx.x * GB_N;
+    const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
     A += b * sA;
     B += b * sB;
     C += b * sC;
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
-    // loader mapping: two float4 per operand per k-tile (rows lr and lr + 64)
-    const int lr = tid >> 2, lk = (tid & 3) * 4;
-    const bool a0ok = i0 + lr < M, a1ok = i0 + lr + 64 < M;
-    const bool b0ok = j0 + lr < N, b1ok = j0 + lr + 64 < N;
-    const float* Ap0 = A + (size_t)(a0ok ? i0 + lr : 0) * lda + lk;
-    const float* Ap1 = A + (size_t)(a1ok ? i0 + lr + 64 : 0) * lda + lk;
-    const float* Bp0 = B + (size_t)(b0ok ? j0 + lr : 0) * ldb + lk;
-    const float* Bp1 = B + (size_t)(b1ok ? j0 + lr + 64 : 0) * ldb + lk;
-    float acc[8][8];
+    // rows past the end read the last one: their outputs are not stored
+    const float4* pa[NA];
+    const float4* pb[NB];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int h = 0; h < NA; h++) {
+        const int e = tid + 128 * h;
+        pa[h] = reinterpret_cast<const float4*>(A + (size_t)min(i0 + e / QK, M - 1) * lda) + e % QK;
+    }
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-
-    float4 ra[2], rb[2];
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    ra[0] = a0ok ? __ldg(reinterpret_cast<const float4*>(Ap0)) : z4;
-    ra[1] = a1ok ? __ldg(reinterpret_cast<const float4*>(Ap1)) : z4;
-    rb[0] = b0ok ? __ldg(reinterpret_cast<const float4*>(Bp0)) : z4;
-    rb[1] = b1ok ? __ldg(reinterpret_cast<const float4*>(Bp1)) : z4;
-    const int nk = Kd / GB_K;
+    for (int h = 0; h < NB; h++) {
+        const int e = tid + 128 * h;
+        pb[h] = reinterpret_cast<const float4*>(B + (size_t)min(j0 + e / QK, N - 1) * ldb) + e % QK;
+    }
+    float4 ra[D][NA], rb[D][NB];
+    auto load = [&](int d) {
+#pragma unroll
+        for (int h = 0; h < NA; h++) {
+            ra[d][h] = __ldg(pa[h]);
+            pa[h] += QK;
+        }
+#pragma unroll
+        for (int h = 0; h < NB; h++) {
+            rb[d][h] = __ldg(pb[h]);
+            pb[h] += QK;
+        }
+    };
+    // f(k) = (k / 4) (32 / QK): the rows a warp stores together are 32 / QK
+    auto store = [&](int buf, int d) {
+#pragma unroll
+        for (int h = 0; h < NA; h++) {
+            const int e = tid + 128 * h, q = e % QK, r = (e / QK) ^ (q * (32 / QK));
+            As[buf][4 * q + 0][r] = ra[d][h].x;
+            As[buf][4 * q + 1][r] = ra[d][h].y;
+            As[buf][4 * q + 2][r] = ra[d][h].z;
+            As[buf][4 * q + 3][r] = ra[d][h].w;
+        }
+#pragma unroll
+        for (int h = 0; h < NB; h++) {
+            const int e = tid + 128 * h, q = e % QK, r = (e / QK) ^ (q * (32 / QK));
+            if (BN * QK % 128 == 0 || e < BN * QK) {
+                Bs[buf][4 * q + 0][r] = rb[d][h].x;
+                Bs[buf][4 * q + 1][r] = rb[d][h].y;
+                Bs[buf][4 * q + 2][r] = rb[d][h].z;
+                Bs[buf][4 * q + 3][r] = rb[d][h].w;
+            }
+        }
+    };
+    uint64_t acc[TM / 2][TN];
+#pragma unroll
+    for (int i = 0; i < TM / 2; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[i][j] = 0ull;
+    const int nk = Kd / BK;
+#pragma unroll
+    for (int d = 0; d < D; d++)
+        if (d < nk) load(d);
+    auto tile = [&](int buf) {
+#pragma unroll
+        for (int kk = 0; kk < BK; kk++) {
+            const int f = (kk >> 2) * (32 / QK);
+            uint64_t a[TM / 2];
+            if (TM >= 4) {
+#pragma unroll
+                for (int i = 0; i < TM / 4; i++) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(
+                        &As[buf][kk][32 * i + ((ty * 4) ^ f)]);
+                    a[2 * i] = v.x;
+                    a[2 * i + 1] = v.y;
+                }
+            } else {
+                a[0] = *reinterpret_cast<const uint64_t*>(&As[buf][kk][(ty * 2) ^ f]);
+            }
+#pragma unroll
+            for (int j = 0; j < TN; j += 2) {
+                if (j + 1 < TN) {
+                    const float2 v = *reinterpret_cast<const float2*>(
+                        &Bs[buf][kk][16 * j + ((2 * tx) ^ f)]);
+                    const uint64_t b0 = pack2(v.x, v.x), b1 = pack2(v.y, v.y);
+#pragma unroll
+                    for (int i = 0; i < TM / 2; i++) {
+                        fma2(acc[i][j], a[i], b0);
+                        fma2(acc[i][j + 1], a[i], b1);
+                    }
+                } else {
+                    const float v = Bs[buf][kk][16 * j + (tx ^ f)];
+                    const uint64_t b0 = pack2(v, v);
+#pragma unroll
+                    for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], a[i], b0);
+                }
+            }
+        }
+    };
     int buf = 0;
-    for (int kt = 0; kt < nk; kt++) {
+    for (int kt = 0; kt < nk; kt += D) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            As[buf][lk + 0][lr + 64 * h] = ra[h].x;
-            As[buf][lk + 1][lr + 64 * h] = ra[h].y;
-            As[buf][lk + 2][lr + 64 * h] = ra[h].z;
-            As[buf][lk + 3][lr + 64 * h] = ra[h].w;
-            Bs[buf][lk + 0][lr + 64 * h] = rb[h].x;
-            Bs[buf][lk + 1][lr + 64 * h] = rb[h].y;
-            Bs[buf][lk + 2][lr + 64 * h] = rb[h].z;
-            Bs[buf][lk + 3][lr + 64 * h] = rb[h].w;
+        for (int d = 0; d < D; d++) {
+            if (kt + d >= nk) break;
+            store(buf, d);
+            __syncthreads();
+            if (kt + d + D < nk) load(d);
+            tile(buf);
+            buf ^= 1;
         }
-        __syncthreads();
-        if (kt + 1 < nk) {
-            const int off = (kt + 1) * GB_K;
-            ra[0] = a0ok ? __ldg(reinterpret_cast<const float4*>(Ap0 + off)) : z4;
-            ra[1] = a1ok ? __ldg(reinterpret_cast<const float4*>(Ap1 + off)) : z4;
-            rb[0] = b0ok ? __ldg(reinterpret_cast<const float4*>(Bp0 + off)) : z4;
-            rb[1] = b1ok ? __ldg(reinterpret_cast<const float4*>(Bp1 + off)) : z4;
-        }
-#pragma unroll
-        for (int kk = 0; kk < GB_K; kk++) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][kk][64 + tx * 4]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-#pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        buf ^= 1;
     }
     // epilogue
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int gi = i0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-        if (gi >= M) continue;
-        const float add = nrm ? nrm[b * sN + gi] : 0.f;
+    for (int j = 0; j < TN; j++) {
+        const int gj = j0 + ((j | 1) < TN ? 16 * (j & ~1) + 2 * tx + (j & 1) : 16 * j + tx);
+        if (gj >= N) continue;
+        size_t col = gj;
+        if (cGroup > 0) {
+            const int l = gj / cGroup;
+            col = (size_t)l * cGroupStride + (gj - l * cGroup);
+        }
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int gj = j0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-            if (gj < N) {
-                size_t off = (size_t)gi * ldc + gj;
-                if (cGroup > 0) {
-                    const int l = gj / cGroup;
-                    off = (size_t)l * cGroupStride + (size_t)gi * ldc + (gj - l * cGroup);
-                }
-                C[off] = fmaf(alpha, acc[i][j], add);
-            }
+        for (int i = 0; i < TM / 2; i++) {
+            const float2 v = unpack2(acc[i][j]);
+            const int gi = i0 + (TM >= 4 ? 32 * (i >> 1) + ty * 4 + 2 * (i & 1) : ty * 2);
+            if (gi < M)
+                C[(size_t)gi * ldc + col] = fmaf(alpha, v.x, nrm ? nrm[b * sN + gi] : 0.f);
+            if (gi + 1 < M)
+                C[(size_t)(gi + 1) * ldc + col] = fmaf(alpha, v.y, nrm ? nrm[b * sN + gi + 1] : 0.f);
         }
     }
 }
@@ -2264,9 +2354,51 @@ cudaError_t launch_gemm_nt_fp32(const float* A, long long sA, int lda, const flo
                                 long long sN, float alpha, cudaStream_t st, int cGroup,
                                 long long cGroupStride)
 {
-    dim3 grid((N + GB_N - 1) / GB_N, (M + GB_M - 1) / GB_M, batch);
-    k_gemm_nt_fp32<<<grid, 256, 0, st>>>(A, sA, lda, B, sB, ldb, M, N, Kd, C, sC, ldc,
-                                          nrm, sN, alpha, cGroup, cGroupStride);
+    // The tile: TN columns a thread, the fewest that cover N in the fewest
+    // column tiles (N = 100 takes 112 columns, not 128); the height that the
+    // cost below prefers.  Measured at 2 x 1,000 x 100: 1.68 ms at TM 16,
+    // 0.96, 0.91, 0.81 at 8, 4, 2; at 6,912 x 16,317: 2.8, 3.0, 3.6, 6.3 ms.
+    const int nt = (N + 127) / 128;
+    const int TN = ((N + nt - 1) / nt + 15) / 16;
+    int TM = 16;
+    long long best = -1;
+    for (int tm = 16; tm >= 2; tm /= 2) {
+        if (Kd % std::min(128 / tm, 32)) break;
+        const long long tiles = (long long)nt * ((M + 8 * tm - 1) / (8 * tm)) * batch;
+        // cycles a step of k, fitted to measured shapes: a tile alone on its
+        // SM waits for its K tiles (lone), tiles together share the FP32
+        // pipes (tm TN) and the shared port (4 (tm + TN))
+        const long long lone = tm == 16  ? 65 + 15 * TN
+                               : tm == 8 ? 30 + 10 * TN
+                               : tm == 4 ? 18 + 10 * TN
+                                         : 14 + 9 * TN;
+        const long long shared = (17 * tm * TN + 40 * (tm + TN)) / 20 + 6;
+        const long long cost = std::max(lone, (tiles + 151) / 152 * shared);
+        if (best < 0 || cost < best) {
+            best = cost;
+            TM = tm;
+        }
+    }
+    dim3 grid(nt, (M + 8 * TM - 1) / (8 * TM), batch);
+#define TG3_FP32_TILE(tm, tn)                                                                    \
+    if (TM == tm && TN == tn)                                                                    \
+    k_gemm_nt_fp32<tm, tn><<<grid, 128, 0, st>>>(A, sA, lda, B, sB, ldb, M, N, Kd, C, sC, ldc, nrm, \
+                                                 sN, alpha, cGroup, cGroupStride)
+#define TG3_FP32_ROWS(tn)                                                                        \
+    TG3_FP32_TILE(16, tn);                                                                       \
+    TG3_FP32_TILE(8, tn);                                                                        \
+    TG3_FP32_TILE(4, tn);                                                                        \
+    TG3_FP32_TILE(2, tn)
+    TG3_FP32_ROWS(1);
+    TG3_FP32_ROWS(2);
+    TG3_FP32_ROWS(3);
+    TG3_FP32_ROWS(4);
+    TG3_FP32_ROWS(5);
+    TG3_FP32_ROWS(6);
+    TG3_FP32_ROWS(7);
+    TG3_FP32_ROWS(8);
+#undef TG3_FP32_ROWS
+#undef TG3_FP32_TILE
     return cudaGetLastError();
 }
 
