@@ -66,174 +66,6 @@ __device__ __forceinline__ float bf(float w, int round = 1)
     return round ? __bfloat162float(__float2bfloat16_rn(w)) : w;
 }
 
-// ---------------------------------------------------------------- conv ---
-// y[n][co][oy][ox] = relu(b[co] + sum_ci,ky,kx W[co][ci][ky][kx] x[n][ci][oy s + ky - 1][ox s + kx - 1])
-// CTA: 16 output channels x 256 output pixels of one image; weights of a
-// 16-channel input slice staged in shared memory.
-__global__ void __launch_bounds__(256)
-k_conv_fwd(const float* __restrict__ x, const float* __restrict__ W, const float* __restrict__ b,
-           float* __restrict__ y, int cin, int cout, int hin, int hout, int stride, int relu,
-           int roundW)
-{
-    __shared__ float ws[16][16][9];
-    const int n = blockIdx.z, co0 = blockIdx.y * 16;
-    const int pix = blockIdx.x * 256 + threadIdx.x;
-    const int oy = pix / hout, ox = pix % hout;
-    const bool valid = pix < hout * hout;
-    float acc[16];
-#pragma unroll
-    for (int c = 0; c < 16; c++) acc[c] = 0.f;
-    const float* xn = x + (size_t)n * cin * hin * hin;
-    for (int ci0 = 0; ci0 < cin; ci0 += 16) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < 16 * 16 * 9; i += 256) {
-            const int c = i / 144, cc = (i / 9) % 16, k = i % 9;
-            ws[c][cc][k] = (co0 + c < cout && ci0 + cc < cin)
-                               ? bf(W[((size_t)(co0 + c) * cin + ci0 + cc) * 9 + k], roundW)
-                               : 0.f;
-        }
-        __syncthreads();
-        if (!valid) continue;
-        const int ncc = min(16, cin - ci0);
-        for (int cc = 0; cc < ncc; cc++) {
-            const float* xc = xn + (size_t)(ci0 + cc) * hin * hin;
-            float v[9];
-#pragma unroll
-            for (int ky = 0; ky < 3; ky++)
-#pragma unroll
-                for (int kx = 0; kx < 3; kx++) {
-                    const int iy = oy * stride + ky - 1, ix = ox * stride + kx - 1;
-                    v[ky * 3 + kx] = (iy >= 0 && iy < hin && ix >= 0 && ix < hin) ? xc[iy * hin + ix] : 0.f;
-                }
-#pragma unroll
-            for (int c = 0; c < 16; c++)
-#pragma unroll
-                for (int k = 0; k < 9; k++) acc[c] = fmaf(ws[c][cc][k], v[k], acc[c]);
-        }
-    }
-    if (!valid) return;
-    for (int c = 0; c < 16 && co0 + c < cout; c++) {
-        float o = acc[c] + b[co0 + c];
-        if (relu) o = fmaxf(o, 0.f);
-        y[(((size_t)n * cout + co0 + c) * hout + oy) * hout + ox] = o;
-    }
-}
-
-// dx[n][ci][iy][ix] = sum_co,ky,kx W[co][ci][ky][kx] dy[n][co][oy][ox] with
-// iy = oy s + ky - 1 (the taps that reached the input pixel).  CTA: 16 input
-// channels x 256 input pixels of one image.
-__global__ void __launch_bounds__(256)
-k_conv_bwd_data(const float* __restrict__ dy, const float* __restrict__ W, float* __restrict__ dx,
-                int cin, int cout, int hin, int hout, int stride, int roundW)
-{
-    __shared__ float ws[16][16][9];   // [co slice][ci][k]
-    const int n = blockIdx.z, ci0 = blockIdx.y * 16;
-    const int pix = blockIdx.x * 256 + threadIdx.x;
-    const int iy = pix / hin, ix = pix % hin;
-    const bool valid = pix < hin * hin;
-    float acc[16];
-#pragma unroll
-    for (int c = 0; c < 16; c++) acc[c] = 0.f;
-    const float* dyn = dy + (size_t)n * cout * hout * hout;
-    for (int co0 = 0; co0 < cout; co0 += 16) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < 16 * 16 * 9; i += 256) {
-            const int c = i / 144, cc = (i / 9) % 16, k = i % 9;
-            ws[c][cc][k] = (co0 + c < cout && ci0 + cc < cin)
-                               ? bf(W[((size_t)(co0 + c) * cin + ci0 + cc) * 9 + k], roundW)
-                               : 0.f;
-        }
-        __syncthreads();
-        if (!valid) continue;
-        const int nc = min(16, cout - co0);
-        for (int c = 0; c < nc; c++) {
-            const float* dc = dyn + (size_t)(co0 + c) * hout * hout;
-#pragma unroll
-            for (int ky = 0; ky < 3; ky++) {
-                const int ty = iy + 1 - ky;
-                if (ty < 0 || ty % stride) continue;
-                const int oy = ty / stride;
-                if (oy >= hout) continue;
-#pragma unroll
-                for (int kx = 0; kx < 3; kx++) {
-                    const int tx = ix + 1 - kx;
-                    if (tx < 0 || tx % stride) continue;
-                    const int ox = tx / stride;
-                    if (ox >= hout) continue;
-                    const float g = dc[oy * hout + ox];
-#pragma unroll
-                    for (int cc = 0; cc < 16; cc++) acc[cc] = fmaf(ws[c][cc][ky * 3 + kx], g, acc[cc]);
-                }
-            }
-        }
-    }
-    if (!valid) return;
-    for (int cc = 0; cc < 16 && ci0 + cc < cin; cc++)
-        dx[(((size_t)n * cin + ci0 + cc) * hin + iy) * hin + ix] = acc[cc];
-}
-
-// dW[co][ci][k] += sum_n,oy,ox dy[n][co][oy][ox] x[n][ci][tap k], db[co] +=
-// sum dy.  CTA: one output channel, 8 input channels, one slice of images;
-// the CTA's partial sums go to the gradient with one atomic add each.
-__global__ void __launch_bounds__(256)
-k_conv_bwd_weight(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dW,
-                  float* __restrict__ db, int N, int cin, int cout, int hin, int hout, int stride,
-                  int imgPerCta)
-{
-    __shared__ float red[72 + 1][8];
-    const int co = blockIdx.x, ci0 = blockIdx.y * 8, n0 = blockIdx.z * imgPerCta;
-    const int nci = min(8, cin - ci0);
-    float acc[8][9];
-    float accb = 0.f;
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-#pragma unroll
-        for (int k = 0; k < 9; k++) acc[c][k] = 0.f;
-    const int P = hout * hout;
-    const int total = min(imgPerCta, N - n0) * P;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        const int n = n0 + e / P, pix = e % P;
-        const int oy = pix / hout, ox = pix % hout;
-        const float g = dy[(((size_t)n * cout + co) * hout + oy) * hout + ox];
-        if (g == 0.f) continue;
-        accb += g;
-        for (int c = 0; c < nci; c++) {
-            const float* xc = x + ((size_t)n * cin + ci0 + c) * hin * hin;
-#pragma unroll
-            for (int ky = 0; ky < 3; ky++)
-#pragma unroll
-                for (int kx = 0; kx < 3; kx++) {
-                    const int iy = oy * stride + ky - 1, ix = ox * stride + kx - 1;
-                    if (iy >= 0 && iy < hin && ix >= 0 && ix < hin)
-                        acc[c][ky * 3 + kx] = fmaf(g, xc[iy * hin + ix], acc[c][ky * 3 + kx]);
-                }
-        }
-    }
-    // block reduction: warp sums, then the 8 warps' sums in order
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            float v = acc[c][k];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) red[c * 9 + k][wid] = v;
-        }
-    for (int o = 16; o > 0; o >>= 1) accb += __shfl_xor_sync(0xffffffffu, accb, o);
-    if (lane == 0) red[72][wid] = accb;
-    __syncthreads();
-    if (threadIdx.x < 73) {
-        float s = 0.f;
-        for (int w = 0; w < 8; w++) s += red[threadIdx.x][w];
-        if (threadIdx.x == 72) {
-            if (blockIdx.y == 0) atomicAdd(db + co, s);
-        } else {
-            const int c = threadIdx.x / 9, k = threadIdx.x % 9;
-            if (c < nci) atomicAdd(dW + ((size_t)co * cin + ci0 + c) * 9 + k, s);
-        }
-    }
-}
-
 // ------------------------------------------------------------ dense ---
 // C[m][n] (+)= sum_k A(m, k) B(k, n); A(m, k) = A[m lda + k] or A[k lda + m]
 // (transA), B(k, n) = B[k ldb + n] or B[n ldb + k] (transB).  Optional bias
@@ -278,6 +110,40 @@ __global__ void k_relu_bwd(float* __restrict__ g, const float* __restrict__ y, s
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x)
         if (!(y[i] > 0.f)) g[i] = 0.f;
+}
+
+// y = max(x + bias, 0) over n rows of cout values
+__global__ void k_bias_relu(float* __restrict__ x, const float* __restrict__ bias, int n, int cout)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * cout; i += gridDim.x * blockDim.x)
+        x[i] = fmaxf(x[i] + bias[i % cout], 0.f);
+}
+
+// out [cols][ldo] = in [rows][cols] transposed, zeros for columns rows .. ldo
+// of out; with round, rounded to bf16; with copy, also the rows as they are.
+__global__ void __launch_bounds__(256)
+k_transpose(const float* __restrict__ in, int rows, int cols, float* __restrict__ out, int ldo,
+            int round, float* __restrict__ copy)
+{
+    __shared__ float t[32][33];
+    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    for (int i = y; i < 32; i += 8) {
+        const bool ok = r0 + i < rows && c0 + x < cols;
+        const float v = ok ? bf(in[(size_t)(r0 + i) * cols + c0 + x], round) : 0.f;
+        t[i][x] = v;
+        if (copy && ok) copy[(size_t)(r0 + i) * cols + c0 + x] = v;
+    }
+    __syncthreads();
+    for (int i = y; i < 32; i += 8)
+        if (c0 + i < cols && r0 + x < ldo) out[(size_t)(c0 + i) * ldo + r0 + x] = t[x][i];
+}
+
+__global__ void k_add(float* __restrict__ a, const float* __restrict__ b, size_t n)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x)
+        a[i] += b[i];
 }
 
 // db[n] += sum_m g[m][n]
@@ -549,19 +415,23 @@ __global__ void k_emb_sim(const float* __restrict__ zp, const float* __restrict_
     S[(size_t)i * n + j] = acc * invTau;
 }
 
-// log-sum-exp of every row (blockIdx.y = 0) and column (1) of S
-__global__ void k_emb_lse(const float* __restrict__ S, int n, float* __restrict__ rowL,
-                          float* __restrict__ colL)
+// log-sum-exp of every row (blockIdx.y = 0) and column (1) of S: a warp each
+// (the FP64 exponentials of one row in one thread took 184 us at n = 256,
+// more than a layer's convolution)
+__global__ void __launch_bounds__(128)
+k_emb_lse(const float* __restrict__ S, int n, float* __restrict__ rowL, float* __restrict__ colL)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= n) return;
     const bool rows = blockIdx.y == 0;
     const size_t st = rows ? 1 : (size_t)n, base = rows ? (size_t)i * n : (size_t)i;
     float m = -INFINITY;
-    for (int k = 0; k < n; k++) m = fmaxf(m, S[base + k * st]);
+    for (int k = lane; k < n; k += 32) m = fmaxf(m, S[base + k * st]);
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     double acc = 0.0;
-    for (int k = 0; k < n; k++) acc += exp((double)(S[base + k * st] - m));
-    (rows ? rowL : colL)[i] = m + (float)log(acc);
+    for (int k = lane; k < n; k += 32) acc += exp((double)(S[base + k * st] - m));
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) (rows ? rowL : colL)[i] = m + (float)log(acc);
 }
 
 // G = dL/dS for L = (1/n) sum_i 0.5 (rowL_i - S_ii) + 0.5 (colL_i - S_ii)
@@ -828,6 +698,12 @@ struct tg3_cnn {
     float* v = nullptr;
     long long step = 0;
     int roundW = 1;             // weights used in bf16 (0: FP32, for gradient checks)
+    // the weights as the FP32 kernels read them (rounded, repacked); stale after
+    // every change of params or roundW
+    float* wtrain = nullptr;
+    size_t wFwd[kLayers] = {}, wBwd[kLayers] = {};
+    bool wStale = true;
+    float* fcT = nullptr;       // wide dense layer's gradient: transposes, its sum
     int cap = 0;                // images the activation buffers hold
     float* act[kLayers + 1] = {};   // act[0] input copy .. act[8] outputs
     float* gact[kLayers + 1] = {};
@@ -848,6 +724,9 @@ struct tg3_cnn {
 
 namespace {
 
+constexpr int kFc = 6;          // the wide dense layer (8192 -> 256)
+inline int pad32(int n) { return (n + 31) / 32 * 32; }
+
 size_t act_size(int l)
 {
     if (l == 0) return 64 * 64;
@@ -866,6 +745,12 @@ int ensure_capacity(tg3_cnn* net, int n)
     }
     cudaFree(net->Rstar);
     cudaFree(net->loss);
+    cudaFree(net->fcT);
+    net->Rstar = net->loss = nullptr;
+    net->fcT = nullptr;
+    net->cap = 0;
+    TG3_CUDA(cudaMalloc(&net->fcT, sizeof(float) * ((size_t)(kShape[kFc].cin + kShape[kFc].cout) *
+                                                        pad32(n) + weight_count(kShape[kFc]))));
     for (int l = 0; l <= kLayers; l++) {
         TG3_CUDA(cudaMalloc(&net->act[l], sizeof(float) * act_size(l) * n));
         TG3_CUDA(cudaMalloc(&net->gact[l], sizeof(float) * act_size(l) * n));
@@ -876,17 +761,55 @@ int ensure_capacity(tg3_cnn* net, int n)
     return TG3_OK;
 }
 
+// The rounded, repacked weights: per convolution the forward and the data
+// gradient's layouts; the wide dense layer's rows and their transpose.
+int repack_weights(tg3_cnn* net)
+{
+    if (!net->wStale) return TG3_OK;
+    cudaStream_t s = net->stream;
+    if (!net->wtrain) {
+        size_t o = 0;
+        for (int l = 0; l <= kFc; l++) {
+            const size_t w = (weight_count(kShape[l]) + 63) / 64 * 64;
+            net->wFwd[l] = o;
+            net->wBwd[l] = o + w;
+            o += 2 * w;
+        }
+        TG3_CUDA(cudaMalloc(&net->wtrain, sizeof(float) * o));
+    }
+    for (int l = 0; l < kFc; l++) {
+        const LayerShape& sh = kShape[l];
+        TG3_CUDA(launch_repack_conv(net->params + net->off[l][0], sh.cin, sh.cout, sh.stride,
+                                    net->roundW, net->wtrain + net->wFwd[l],
+                                    l ? net->wtrain + net->wBwd[l] : nullptr, s));
+    }
+    const LayerShape& f = kShape[kFc];
+    k_transpose<<<dim3(f.cin / 32, f.cout / 32), 256, 0, s>>>(
+        net->params + net->off[kFc][0], f.cout, f.cin, net->wtrain + net->wBwd[kFc], f.cout,
+        net->roundW, net->wtrain + net->wFwd[kFc]);
+    TG3_LAUNCH_CHECK("weights repack");
+    net->wStale = false;
+    return TG3_OK;
+}
+
 int forward(tg3_cnn* net, int n)
 {
     cudaStream_t s = net->stream;
+    int st = repack_weights(net);
+    if (st) return st;
     for (int l = 0; l < kLayers; l++) {
         const LayerShape& sh = kShape[l];
         const float* W = net->params + net->off[l][0];
         const float* b = net->params + net->off[l][1];
         if (sh.stride) {
-            dim3 grid((sh.hout * sh.hout + 255) / 256, (sh.cout + 15) / 16, n);
-            k_conv_fwd<<<grid, 256, 0, s>>>(net->act[l], W, b, net->act[l + 1], sh.cin, sh.cout,
-                                             sh.hin, sh.hout, sh.stride, 1, net->roundW);
+            TG3_CUDA(launch_conv_fwd(l, net->act[l], net->wtrain + net->wFwd[l], b,
+                                     net->act[l + 1], n, sh.cin, sh.cout, s));
+        } else if (l == kFc) {
+            TG3_CUDA(launch_gemm_nt_fp32(net->act[l], 0, sh.cin, net->wtrain + net->wFwd[l], 0,
+                                         sh.cin, n, sh.cout, sh.cin, 1, net->act[l + 1], 0, sh.cout,
+                                         nullptr, 0, 1.f, s));
+            k_bias_relu<<<cnn_grid((size_t)n * sh.cout, 256), 256, 0, s>>>(net->act[l + 1], b, n,
+                                                                           sh.cout);
         } else {
             dim3 grid((sh.cout + 15) / 16, (n + 15) / 16);
             k_dense<<<grid, dim3(16, 16), 0, s>>>(net->act[l], W, net->act[l + 1], n, sh.cout,
@@ -898,7 +821,9 @@ int forward(tg3_cnn* net, int n)
     return TG3_OK;
 }
 
-// gact[kLayers] holds dL/d outputs; fills grads (accumulating)
+// gact[kLayers] holds dL/d outputs; fills grads (accumulating).  Gradients
+// with respect to a ReLU's output are zeroed where it is not positive: by
+// the convolutions' data gradient itself, after the dense layers by k_relu_bwd.
 int backward(tg3_cnn* net, int n)
 {
     cudaStream_t s = net->stream;
@@ -908,21 +833,32 @@ int backward(tg3_cnn* net, int n)
         float* dW = net->grads + net->off[l][0];
         float* db = net->grads + net->off[l][1];
         float* gy = net->gact[l + 1];
-        // through this layer's ReLU (all but the last)
-        if (l < kLayers - 1) {
+        if (l == kFc || l == kFc - 1) {
             const size_t cnt = act_size(l + 1) * n;
             k_relu_bwd<<<cnn_grid(cnt, 256), 256, 0, s>>>(gy, net->act[l + 1], cnt);
         }
         if (sh.stride) {
-            const int imgPerCta = 8;
-            dim3 gw(sh.cout, (sh.cin + 7) / 8, (n + imgPerCta - 1) / imgPerCta);
-            k_conv_bwd_weight<<<gw, 256, 0, s>>>(net->act[l], gy, dW, db, n, sh.cin, sh.cout,
-                                                  sh.hin, sh.hout, sh.stride, imgPerCta);
-            if (l > 0) {
-                dim3 gd((sh.hin * sh.hin + 255) / 256, (sh.cin + 15) / 16, n);
-                k_conv_bwd_data<<<gd, 256, 0, s>>>(gy, W, net->gact[l], sh.cin, sh.cout, sh.hin,
-                                                    sh.hout, sh.stride, net->roundW);
-            }
+            TG3_CUDA(launch_conv_bwd_weight(l, net->act[l], gy, dW, db, n, sh.cin, sh.cout, s));
+            if (l > 0)
+                TG3_CUDA(launch_conv_bwd_data(l, gy, net->wtrain + net->wBwd[l], net->act[l],
+                                              net->gact[l], n, sh.cin, sh.cout, s));
+        } else if (l == kFc) {
+            // dW[o][i] += sum_n gy[n][o] x[n][i] and dx = gy W, both as products of rows
+            const int np = pad32(n);
+            float* xT = net->fcT;
+            float* gT = xT + (size_t)sh.cin * np;
+            float* sum = gT + (size_t)sh.cout * np;
+            k_transpose<<<dim3(sh.cin / 32, np / 32), 256, 0, s>>>(net->act[l], n, sh.cin, xT, np, 0,
+                                                                  nullptr);
+            k_transpose<<<dim3(sh.cout / 32, np / 32), 256, 0, s>>>(gy, n, sh.cout, gT, np, 0,
+                                                                   nullptr);
+            TG3_CUDA(launch_gemm_nt_fp32(gT, 0, np, xT, 0, np, sh.cout, sh.cin, np, 1, sum, 0,
+                                         sh.cin, nullptr, 0, 1.f, s));
+            k_add<<<cnn_grid(weight_count(sh), 256), 256, 0, s>>>(dW, sum, weight_count(sh));
+            k_col_sum<<<(sh.cout + 255) / 256, 256, 0, s>>>(gy, db, n, sh.cout);
+            TG3_CUDA(launch_gemm_nt_fp32(gy, 0, sh.cout, net->wtrain + net->wBwd[l], 0, sh.cout, n,
+                                         sh.cin, sh.cout, 1, net->gact[l], 0, sh.cin, nullptr, 0,
+                                         1.f, s));
         } else {
             // dW[o][i] += sum_n gy[n][o] x[n][i]; db[o] += sum_n gy[n][o]; dx = gy W
             dim3 g1((sh.cin + 15) / 16, (sh.cout + 15) / 16);
@@ -1007,6 +943,8 @@ extern "C" int tg3_cnn_destroy(tg3_cnn* net)
     }
     cudaFree(net->Rstar);
     cudaFree(net->loss);
+    cudaFree(net->wtrain);
+    cudaFree(net->fcT);
     cudaFree(net->emb);
     cudaFree(net->embLoss);
     cudaFree(net->tcW);
@@ -1032,6 +970,7 @@ extern "C" int tg3_cnn_params(tg3_cnn* net, float* host, int set)
     TG3_CUDA(cudaMemcpy(set ? (void*)net->params : (void*)host, set ? (const void*)host : net->params,
                         sizeof(float) * net->nParams,
                         set ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
+    if (set) net->wStale = true;
     return TG3_OK;
 }
 
@@ -1100,6 +1039,7 @@ extern "C" int tg3_cnn_adam(tg3_cnn* net, float lr)
     if (!net) return fail(TG3_ERR_ARG, "null network");
     TG3_CUDA(cudaSetDevice(net->device));
     net->step++;
+    net->wStale = true;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)net->step), c2 = 1.f - powf(b2, (float)net->step);
     k_adam<<<cnn_grid(net->nParams, 256), 256, 0, net->stream>>>(net->params, net->grads, net->m,
@@ -1113,6 +1053,7 @@ extern "C" int tg3_cnn_set_bf16(tg3_cnn* net, int enable)
 {
     if (!net) return fail(TG3_ERR_ARG, "null network");
     net->roundW = enable != 0;
+    net->wStale = true;
     return TG3_OK;
 }
 
@@ -1185,7 +1126,7 @@ extern "C" int tg3_cnn_contrastive(tg3_cnn* net, const float* outP, const float*
     k_emb_norm<<<(n + 7) / 8, 256, 0, s>>>(outP, n, zp, invP);
     k_emb_norm<<<(n + 7) / 8, 256, 0, s>>>(outR, n, zr, invR);
     k_emb_sim<<<dim3((n + 127) / 128, n), 128, 0, s>>>(zp, zr, n, invTau, S);
-    k_emb_lse<<<dim3((n + 127) / 128, 2), 128, 0, s>>>(S, n, rowL, colL);
+    k_emb_lse<<<dim3((n + 3) / 4, 2), 128, 0, s>>>(S, n, rowL, colL);
     k_emb_dS<<<dim3((n + 127) / 128, n), 128, 0, s>>>(S, rowL, colL, n, G);
     k_emb_grad<<<dim3(n, 2), kEmb, 0, s>>>(G, zp, zr, invP, invR, outP, tstar, n, invTau, S, rowL,
                                            colL, dOutP, dOutR, net->embLoss);

@@ -534,4 +534,16 @@ cudaError_t launch_match_propose_classes(const float* out, int n, const RefView*
                                          const int* cls, int maxRef, int nRot, int nTrans,
                                          unsigned long long seed, double* quat, double* trans,
                                          int* idx, cudaStream_t st);
+
+// The pose network's FP32 convolutions (tg3_cnn_train.cu), by layer 0 .. 5,
+// on weights repacked by launch_repack_conv (fwd: [cin 9][cout]; bwd: the
+// data gradient's layout, as many floats; either may be null).
+cudaError_t launch_repack_conv(const float* W, int cin, int cout, int stride, int round, float* fwd,
+                               float* bwd, cudaStream_t st);
+cudaError_t launch_conv_fwd(int layer, const float* x, const float* wt, const float* bias, float* y,
+                            int n, int cin, int cout, cudaStream_t st);
+cudaError_t launch_conv_bwd_data(int layer, const float* dy, const float* wt, const float* act,
+                                 float* dx, int n, int cin, int cout, cudaStream_t st);
+cudaError_t launch_conv_bwd_weight(int layer, const float* x, const float* dy, float* dW, float* db,
+                                   int n, int cin, int cout, cudaStream_t st);
 }  // namespace tg3

@@ -2354,32 +2354,34 @@ cudaError_t launch_gemm_nt_fp32(const float* A, long long sA, int lda, const flo
                                 long long sN, float alpha, cudaStream_t st, int cGroup,
                                 long long cGroupStride)
 {
-    // The tile: TN columns a thread, the fewest that cover N in the fewest
-    // column tiles (N = 100 takes 112 columns, not 128); the height that the
-    // cost below prefers.  Measured at 2 x 1,000 x 100: 1.68 ms at TM 16,
-    // 0.96, 0.91, 0.81 at 8, 4, 2; at 6,912 x 16,317: 2.8, 3.0, 3.6, 6.3 ms.
-    const int nt = (N + 127) / 128;
-    const int TN = ((N + nt - 1) / nt + 15) / 16;
-    int TM = 16;
+    // The tile that the cost below prefers: N = 100 takes 112 columns, not 128,
+    // and small problems take small tiles.  Measured at 2 x 1,000 x 100: 1.68 ms
+    // at TM 16, 0.96, 0.91, 0.81 at 8, 4, 2; at 6,912 x 16,317: 2.8, 3.0, 3.6,
+    // 6.3 ms.
+    int TM = 16, TN = 8;
     long long best = -1;
     for (int tm = 16; tm >= 2; tm /= 2) {
         if (Kd % std::min(128 / tm, 32)) break;
-        const long long tiles = (long long)nt * ((M + 8 * tm - 1) / (8 * tm)) * batch;
-        // cycles a step of k, fitted to measured shapes: a tile alone on its
-        // SM waits for its K tiles (lone), tiles together share the FP32
-        // pipes (tm TN) and the shared port (4 (tm + TN))
-        const long long lone = tm == 16  ? 65 + 15 * TN
-                               : tm == 8 ? 30 + 10 * TN
-                               : tm == 4 ? 18 + 10 * TN
-                                         : 14 + 9 * TN;
-        const long long shared = (17 * tm * TN + 40 * (tm + TN)) / 20 + 6;
-        const long long cost = std::max(lone, (tiles + 151) / 152 * shared);
-        if (best < 0 || cost < best) {
-            best = cost;
-            TM = tm;
+        for (int tn = 8; tn >= 1; tn--) {
+            const long long tiles =
+                (long long)((N + 16 * tn - 1) / (16 * tn)) * ((M + 8 * tm - 1) / (8 * tm)) * batch;
+            // cycles a step of k, fitted to measured shapes: a tile alone on
+            // its SM waits for its K tiles (lone), tiles together share the
+            // FP32 pipes (tm tn) and the shared port (4 (tm + tn))
+            const long long lone = tm == 16  ? 65 + 15 * tn
+                                   : tm == 8 ? 30 + 10 * tn
+                                   : tm == 4 ? 18 + 10 * tn
+                                             : 14 + 9 * tn;
+            const long long shared = (17 * tm * tn + 40 * (tm + tn)) / 20 + 6;
+            const long long cost = std::max(lone, (tiles + 151) / 152 * shared);
+            if (best < 0 || cost < best) {
+                best = cost;
+                TM = tm;
+                TN = tn;
+            }
         }
     }
-    dim3 grid(nt, (M + 8 * TM - 1) / (8 * TM), batch);
+    dim3 grid((N + 16 * TN - 1) / (16 * TN), (M + 8 * TM - 1) / (8 * TM), batch);
 #define TG3_FP32_TILE(tm, tn)                                                                    \
     if (TM == tm && TN == tn)                                                                    \
     k_gemm_nt_fp32<tm, tn><<<grid, 128, 0, st>>>(A, sA, lda, B, sB, ldb, M, N, Kd, C, sC, ldc, nrm, \
