@@ -284,6 +284,7 @@ extern "C" int tg3_ctx_create(tg3_ctx** out, int device)
     if (e == cudaSuccess) e = cudaMemset(c->d_flag, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&c->d_volTable, sizeof(float4*) * kMaxClasses);
     if (e == cudaSuccess) e = cudaMemset(c->d_volTable, 0, sizeof(float4*) * kMaxClasses);
+    if (e == cudaSuccess) e = prefer_carveouts();
     if (e != cudaSuccess) {
         int st = cuda_fail(e, "context set-up");
         tg3_ctx_destroy(c);
@@ -2024,6 +2025,11 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                       : (float*)ws_get(c, WS_PROJ, sizeof(float) * project_scratch_floats(nR, Kp),
                                        &st);
     if (!img2 && !pbank && !pscr) return st;
+    int* best = nullptr;
+    if (split && !c->scanPair) {
+        best = (int*)ws_get(c, WS_BEST, sizeof(int) * (size_t)IB * std::max(nK, 16), &st);
+        if (!best) return st;
+    }
     cudaStream_t s = c->stream;
     const long long splitP = split ? (long long)nRt * Kp : 0;
     {
@@ -2069,6 +2075,14 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
         const float* cc = ctf + (size_t)l0 * K;
         const float* ss = sigRcp + (size_t)l0 * K;
         const long long splitA = split ? (long long)n * nT * Kp : 0;
+        // few images of one class (its fallback particles): each image's
+        // rotations over several CTAs of the weights kernel, so the GPU fills
+        int nc = 1;
+        if (nK == 1 && n < 2 * 152 && nR >= 512)
+            nc = std::min(std::min(16, nR / 256), (2 * 152 + n - 1) / n);
+        // every weights block's largest log-likelihood comes with the split cross
+        // term, so the weights kernel reads D once
+        TileBest tb = {best, nK > 1 ? nR : (nR + nc - 1) / nc, nK > 1 ? nK : nc, nrmG, n};
         {
             StageTimer tm(c, TG3_STAGE_SHIFT);
             TG3_CUDA(launch_shift_bank(dd, cc, ss, nullptr, bank, n, nT, 1, nullptr, nullptr, K, A,
@@ -2100,6 +2114,9 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
             StageTimer tm(c, TG3_STAGE_CROSS);
             // the cross term is written image-major: D[l][r][t]
             const int cols = n * nT;
+            if (best) {
+                TG3_CUDA(launch_fill_int(best, (size_t)n * tb.groups, kFloatKeyNegInf, s));
+            }
             if (split) {
                 const int Nt = std::min(c->scanTileN > 0 ? c->scanTileN : 256,
                                         (cols + 15) / 16 * 16);
@@ -2107,7 +2124,8 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                 TG3_CUDA(launch_gemm_bf16x3(P, nRt, A, (long long)cols, nRt, Nt, Kp, items, 0, Nt,
                                             cols, D, 0, nT, nullptr, 0, -2.0f, c->d_flag, s, nT,
                                             (long long)nRt * nT, c->scanPair != 0,
-                                            Kp % c->scanBK == 0 ? c->scanBK : 64));
+                                            Kp % c->scanBK == 0 ? c->scanBK : 64,
+                                            best ? &tb : nullptr));
             } else {
                 TG3_CUDA(launch_gemm_nt_fp32(P, 0, Kp, A, 0, Kp, nRt, cols, Kp, 1, D, 0, nT,
                                              nullptr, 0, -2.0f, s, nT, (long long)nRt * nT));
@@ -2116,11 +2134,6 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
         {
             StageTimer tm(c, TG3_STAGE_WEIGHTS);
             if (nK == 1) {
-                // few images (the fallback particles of one class): each
-                // image's rotations over several CTAs, so the GPU fills
-                int nc = 1;
-                if (n < 2 * 152 && nR >= 512)
-                    nc = std::min(std::min(16, nR / 256), (2 * 152 + n - 1) / n);
                 double* tmp = nullptr;
                 if (nc > 1) {
                     tmp = (double*)ws_get(c, WS_WCHUNK,
@@ -2131,7 +2144,7 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                                         pR, 0, pT, 0, nullptr, wC + l0, wR + (size_t)l0 * nR,
                                         wT + (size_t)l0 * nT, baseL + l0,
                                         dvp ? dvp + (size_t)l0 * nR * nT : nullptr, s, 512, nc,
-                                        tmp));
+                                        tmp, best));
             } else {
                 // one block per (image, class): D[l][k nR + r][t] is block l nK + k
                 const size_t b0 = (size_t)l0 * nK;
@@ -2142,7 +2155,8 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                                         x0r, pR, 0, pT, 0, nullptr, wC + b0, wR + b0 * nR,
                                         wT + b0 * nT, baseL + b0,
                                         dvp ? dvp + b0 * nR * nT : nullptr, s,
-                                        nR < 128 ? 128 : (nR < 256 ? 256 : 512)));
+                                        nR < 128 ? 128 : (nR < 256 ? 256 : 512), 1, nullptr,
+                                        best));
             }
         }
     }

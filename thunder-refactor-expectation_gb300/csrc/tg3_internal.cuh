@@ -41,6 +41,15 @@ int cuda_fail(cudaError_t e, const char* what);
         if (e_ != cudaSuccess) return ::tg3::cuda_fail(e_, what);        \
     } while (0)
 
+// A float as an int in the same order (its own inverse on the way back); NaN
+// aside, the largest of floats is the largest of keys.
+__host__ __device__ __forceinline__ int float_key_bits(int b) { return b ^ ((b >> 31) & 0x7fffffff); }
+#ifdef __CUDACC__
+__device__ __forceinline__ int float_key(float x) { return float_key_bits(__float_as_int(x)); }
+__device__ __forceinline__ float key_float(int k) { return __int_as_float(float_key_bits(k)); }
+#endif
+constexpr int kFloatKeyNegInf = (int)(0xff800000u ^ 0x7fffffffu);
+
 inline size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
 // ------------------------------------------------- projection volume layout --
@@ -94,6 +103,7 @@ enum WsSlot {
     WS_SPLITK,       // split-K partial sums of the global search's norm term
     WS_WCHUNK,       // per-chunk weights of a row-split weights launch
     WS_RECO2D,       // 2-D reconstruction: accumulator, staged F / T, image
+    WS_BEST,         // global search: the largest log-likelihood of every weights block
     WS_COUNT
 };
 
@@ -347,7 +357,7 @@ cudaError_t launch_weights(const float* D, long long sD, int ldc, int nR,
                            long long sT, const double* pwC, double* wC,
                            double* wR, double* wT, double* base, float* dvp,
                            cudaStream_t st, int threads = 512, int nc = 1,
-                           double* chunkTmp = nullptr);
+                           double* chunkTmp = nullptr, const int* best = nullptr);
 // doubles of chunkTmp launch_weights needs for nBlocks items of nc chunks
 inline size_t weights_chunk_doubles(int nBlocks, int nc, int nT)
 {
@@ -500,12 +510,33 @@ cudaError_t launch_gemm_nt_bf16x3(const float* A, long long sA, int lda,
 size_t bf16x3_scratch_bytes(int M, int N, int Kd, int batch);
 // General split-bf16 GEMM over `items` (see tg3_tc.cu): A/B point at hi
 // planes followed by lo planes of rowsA / rowsB rows of Kd bf16 elements.
+// With best (column groups only), key[l groups + row / rows] receives the
+// largest C + nrm[row nrmStride + l] of column group l and each group of rows,
+// as float_key; the caller sets the keys to float_key(-inf) first.
+// besideProjections: keep to 131 KB of shared memory.  An SM's split between
+// shared memory and L1 changes only while the SM is idle, so a projection that
+// starts on SMs where another stream's kernel still runs keeps that kernel's
+// split to its end: 3.9 ms at up to 64 KB of shared memory, 4.1 at 132, 4.6 at
+// 164, 7.8 above.  Three contexts' local phases in turn take 5.1 ms each with
+// the GEMM, the shift bank and the resampling kept so (prefer_carveouts), 6.2
+// to 7.0 ms without; alone the GEMM's third stage was worth 0.16 of 5.2 ms.
+struct TileBest {
+    int* key;
+    int rows, groups;
+    const float* nrm;
+    int nrmStride;
+};
 cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, long long rowsB,
                                int M, int N, int Kd, int items, int aRowsPerItem,
                                int bRowsPerItem, int nTotal, float* C, long long sC, int ldc,
                                const float* nrm, long long sN, float alpha, int* flag,
                                cudaStream_t st, int cGroup = 0, long long cGroupStride = 0,
-                               bool pair = false, int bk = 64);
+                               bool pair = false, int bk = 64, const TileBest* best = nullptr,
+                               bool besideProjections = false);
+// Shared-memory preferences of the kernels that run beside projections, for
+// the current device.
+cudaError_t prefer_carveouts();
+cudaError_t launch_fill_int(int* p, size_t n, int value, cudaStream_t st);
 
 }  // namespace tg3
 

@@ -1316,7 +1316,7 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
           const double* __restrict__ pwR, long long sR,
           const double* __restrict__ pwT, long long sT, const double* __restrict__ pwC,
           double* __restrict__ wC, double* __restrict__ wR, double* __restrict__ wT,
-          double* __restrict__ base, float* __restrict__ dvp, int nc)
+          double* __restrict__ base, float* __restrict__ dvp, int nc, const int* __restrict__ best)
 {
     extern __shared__ float wsm[];
     float* wTs = wsm;                // [nT]
@@ -1345,9 +1345,10 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
         wTs[t] = 0.f;
         pTs[t] = (float)pt[t];
     }
-    // pass 1: maximum (four rows per warp in flight)
+    // pass 1: maximum (four rows per warp in flight), unless the GEMM that wrote
+    // D found it
     float mx = -CUDART_INF_F;
-    for (int r0 = wid; r0 < nR; r0 += 4 * nw) {
+    for (int r0 = wid; r0 < nR && !best; r0 += 4 * nw) {
         float v[4][TS > 0 ? TS : 1];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -1376,7 +1377,7 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
         if (lane == 0) redf[0] = v;
     }
     __syncthreads();
-    const float M = redf[0];
+    const float M = best ? key_float(best[blk]) : redf[0];
     const double x0b = x0 ? x0[item] : 0.0;
     // pass 2: marginals
     float tacc[TS > 0 ? TS : 1], ptv[TS > 0 ? TS : 1];
@@ -1387,11 +1388,13 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
         ptv[j] = (TS > 0 && t < nT) ? pTs[t] : 0.f;
     }
     float cacc = 0.f;
-    // two rows per warp in flight: both rows' loads precede their arithmetic
-    for (int r0 = wid; r0 < nR; r0 += 2 * nw) {
-        float dv[2][TS > 0 ? TS : 1], prr[2], ad[2];
+    // four rows per warp in flight: their loads precede their arithmetic, and
+    // their sums over the lanes share the steps of one reduction
+    const bool b4 = lane & 16, b3 = lane & 8;
+    for (int r0 = wid; r0 < nR; r0 += 4 * nw) {
+        float dv[4][TS > 0 ? TS : 1], prr[4], ad[4], racc[4];
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
+        for (int q = 0; q < 4; q++) {
             const int r = r0 + q * nw;
             const bool rok = r < nR;
             prr[q] = rok ? (float)pr[r] : 0.f;
@@ -1404,11 +1407,11 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
             }
         }
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
+        for (int q = 0; q < 4; q++) {
             const int r = r0 + q * nw;
-            if (r >= nR) break;
+            racc[q] = 0.f;
+            if (r >= nR) continue;
             const float* row = Db + (size_t)r * ldc;
-            float racc = 0.f;
             if (TS > 0) {
 #pragma unroll
                 for (int j = 0; j < (TS > 0 ? TS : 1); j++) {
@@ -1416,7 +1419,7 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
                     if (t < nT) {
                         const float d = dv[q][j] + ad[q];
                         const float sv = __expf(d - M);
-                        racc = fmaf(sv, ptv[j], racc);
+                        racc[q] = fmaf(sv, ptv[j], racc[q]);
                         tacc[j] = fmaf(sv, prr[q], tacc[j]);
                         if (dvp)
                             dvp[((size_t)item * nRall + r0c + r) * nT + t] =
@@ -1427,17 +1430,29 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
                 for (int t = lane; t < nT; t += 32) {
                     const float d = row[t] + ad[q];
                     const float sv = __expf(d - M);
-                    racc = fmaf(sv, pTs[t], racc);
+                    racc[q] = fmaf(sv, pTs[t], racc[q]);
                     atomicAdd(wTs + t, sv * prr[q]);
                     if (dvp)
                         dvp[((size_t)item * nRall + r0c + r) * nT + t] =
                             (float)(x0b + (double)d);
                 }
             }
-            racc = warp_sum(racc);
-            cacc = fmaf(racc, prr[q], cacc);   // sum_t s pT[t] pR[r], once per row
-            if (lane == 0) wR[(size_t)item * nRall + r0c + r] = (double)racc * pc;
         }
+        // the four butterfly sums (the same additions as one after another):
+        // a lane keeps two rows after the first step, one after the second;
+        // lanes 8 q .. 8 q + 7 end with row q's
+        float s0 = (b4 ? racc[2] : racc[0]) + __shfl_xor_sync(0xffffffffu, b4 ? racc[0] : racc[2], 16);
+        float s1 = (b4 ? racc[3] : racc[1]) + __shfl_xor_sync(0xffffffffu, b4 ? racc[1] : racc[3], 16);
+        float sr = (b3 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b3 ? s0 : s1, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, o);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float rs = __shfl_sync(0xffffffffu, sr, 8 * q);
+            if (r0 + q * nw < nR) cacc = fmaf(rs, prr[q], cacc);   // sum_t s pT[t] pR[r], once per row
+        }
+        const int rw = r0 + (lane >> 3) * nw;
+        if ((lane & 7) == 0 && rw < nR) wR[(size_t)item * nRall + r0c + rw] = (double)sr * pc;
     }
     if (TS > 0) {
 #pragma unroll
@@ -2624,6 +2639,19 @@ __global__ void k_sum_parts(const float* __restrict__ part, int S, size_t cnt,
     }
 }
 
+__global__ void k_fill_int(int* __restrict__ p, size_t n, int value)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x)
+        p[i] = value;
+}
+
+cudaError_t launch_fill_int(int* p, size_t n, int value, cudaStream_t st)
+{
+    k_fill_int<<<grid_for(n, 256), 256, 0, st>>>(p, n, value);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_sum_parts(const float* part, int S, size_t cnt, float* out, cudaStream_t st)
 {
     if (S < 1) return cudaErrorInvalidValue;
@@ -2667,7 +2695,8 @@ cudaError_t launch_weights(const float* D, long long sD, int ldc, int nR, int nT
                            const double* pwR,
                            long long sR, const double* pwT, long long sT, const double* pwC,
                            double* wC, double* wR, double* wT, double* base, float* dvp,
-                           cudaStream_t st, int threads, int nc, double* chunkTmp)
+                           cudaStream_t st, int threads, int nc, double* chunkTmp,
+                           const int* best)
 {
     if (nc < 1 || (nc > 1 && (G != 1 || !chunkTmp))) return cudaErrorInvalidValue;
     if (threads != 128 && threads != 256 && threads != WEIGHTS_THREADS)
@@ -2681,7 +2710,7 @@ cudaError_t launch_weights(const float* D, long long sD, int ldc, int nR, int nT
 #define TG3_WEIGHTS(TS)                                                                        \
     k_weights<TS><<<nBlocks * nc, threads, smem, st>>>(D, sD, ldc, nR, nT, G, nrmG, nrmRS, x0, \
                                                        pwR, sR, pwT, sT, pwC, cC, wR, cT, cB,  \
-                                                       dvp, nc)
+                                                       dvp, nc, best)
     if (nT <= 32) TG3_WEIGHTS(1);
     else if (nT <= 64) TG3_WEIGHTS(2);
     else if (nT <= 128) TG3_WEIGHTS(4);
@@ -2771,6 +2800,17 @@ cudaError_t launch_nrm_classes(const float* nrm, int nK, int nR, int n, float* o
 {
     k_nrm_classes<<<grid_for((size_t)nK * nR * n, 256), 256, 0, st>>>(nrm, nK, nR, n, out);
     return cudaGetLastError();
+}
+
+cudaError_t prefer_carveouts()
+{
+    // half of the SM's memory as L1: their own full occupancy would take up to
+    // 200 KB as shared memory (8 CTAs of 25 KB)
+    cudaError_t e = cudaFuncSetAttribute(k_shift_bank, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         50);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_resample, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
+    return e;
 }
 
 cudaError_t launch_resample(int nP, int n, const double* u, const double* w, const int* perm,

@@ -5,11 +5,17 @@
 // the product formed as Ah Bh + Ah Bl + Al Bh (the lo x lo term, ~2^-16 of
 // the product, is dropped), accumulated in FP32 in tensor memory.
 //
-// One CTA per (128-row tile of A, batch item); N (<= 256) columns in one
-// UMMA of shape 128 x N x 16.  128 threads:
-//   warp 0 lane 0 : TMA producer (cp.async.bulk.tensor, 128B swizzle),
+// A tile is (128 rows of A, batch item); N (<= 256) columns in one UMMA of
+// shape 128 x N x 16.  One CTA an SM walks the tiles, 320 threads:
+//   warp 0 lane 0 : TMA producer (cp.async.bulk.tensor),
 //   warp 1 lane 0 : tcgen05.mma issuer, commits to the stage's empty barrier,
-//   warps 0-3     : epilogue (tcgen05.ld 32x32b, + nrm, store).
+//   warps 2-9     : epilogue (tcgen05.ld 32x32b, + nrm, store), two warps to a
+//                   quarter of the rows, alternate 32 columns each.
+// Two accumulators in tensor memory: while the epilogue drains one, the MMAs
+// of the next tile fill the other and the copies run ahead of both.  (With a
+// CTA per tile the set-up, the pipeline's fill and the epilogue stood between
+// the tiles' products: 4.8 ms for 6,912 x 98,000 x 768, the short K of a box-64
+// search, where they are most of a tile; now 2.1 ms, 1.5 PFLOP/s executed.)
 // Every mbarrier wait is bounded (clock64 budget); on expiry the CTA records
 // TG3 flag bit 4, stops issuing, waits (bounded) for its own copies and MMAs,
 // frees its tensor memory and returns.
@@ -17,6 +23,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "tg3_internal.cuh"
 #include "tg3_tcgen05.cuh"
@@ -29,7 +37,12 @@ using namespace tc;
 
 constexpr int TC_M = 128;          // rows of A per CTA (UMMA M)
 constexpr int TC_BK = 64;          // bf16 elements per K block (one 128-byte row)
-constexpr int TC_THREADS = 128;
+constexpr int TC_EPI = 8;            // epilogue warps
+constexpr int TC_THREADS = 64 + 32 * TC_EPI;
+constexpr int TC_PITCH = 36;         // row pitch of the transposition buffer (16-byte rows, no conflicts)
+constexpr int TC_SEGS = 8;           // column groups of a tile whose norms are fetched ahead
+constexpr int TC_ROWS = 8;           // rows of it
+constexpr int TC_STAGE = TC_ROWS * TC_PITCH;
 struct TcParams {
     int M, N, Kd;            // rows of A per item, columns (rows of B) per item, K
     int aRowsPerItem;        // A row offset between items (0: A shared by all items)
@@ -48,6 +61,14 @@ struct TcParams {
     long long sN;
     float alpha;
     int* flag;
+    // with best: the largest C + norm of every (column group, group of rows),
+    // as ordered ints (float_key): best[l bestGroups + row / bestRows], the norm
+    // of row r in column group l at bestNrm[r bestNs + l]
+    int* best;
+    int bestRows, bestGroups;
+    const float* bestNrm;
+    int bestNs;
+    int mTiles, tiles;       // row tiles of an item, tiles of the problem
 };
 
 // K-major operand descriptors: 128-byte rows with the 128-byte swizzle
@@ -57,6 +78,123 @@ template <int BK>
 __device__ __forceinline__ uint64_t desc(uint32_t saddr)
 {
     return BK == 64 ? umma_desc(saddr) : umma_desc_sw64(saddr);
+}
+
+// The norms that a warp's rows need for the tile's first TC_SEGS column
+// groups, lane = row, fetched before the tile's products are waited for.
+__device__ __forceinline__ void load_norms(const TcParams& p, float* ad, int lane, int rowBase,
+                                           int item, int nValid)
+{
+    const int j0 = item * p.colPerItem;
+    const int l0 = j0 / p.cGroup, l1 = (j0 + nValid - 1) / p.cGroup;
+    const float* src = p.bestNrm + (size_t)min(rowBase + lane, p.M - 1) * p.bestNs + l0;
+    for (int k = 0; k < min(l1 - l0 + 1, TC_SEGS); k++) ad[k * 32 + lane] = src[k];
+}
+
+// Largest value of each of the chunk's column groups (columns c0 .. c0 + cn - 1
+// of the tile, v[] of this lane's row) with the row's norm, then over the
+// warp's rows of every row group, into best.  fl(x + norm) grows with x, so the
+// norm is added to the largest x only.
+__device__ __forceinline__ void chunk_best(const TcParams& p, const float* v, int cn, const float* ad,
+                                           int lane, int rowBase, int rows, int j0, int c0)
+{
+    const bool rowOk = lane < rows;
+    const int row = rowBase + lane;
+    const int g0 = rowBase / p.bestRows, g1 = (rowBase + rows - 1) / p.bestRows;
+    const int g = rowOk ? row / p.bestRows : -1;
+    const int lTile = j0 / p.cGroup;
+    int l = (j0 + c0) / p.cGroup;
+    auto put = [&](float m) {                                   // m: group l's largest of the row
+        const float n = l - lTile < TC_SEGS ? ad[(l - lTile) * 32 + lane]
+                                            : p.bestNrm[(size_t)min(row, p.M - 1) * p.bestNs + l];
+        const int key = float_key(m + n);
+        for (int k = g0; k <= g1; k++) {
+            const int top = __reduce_max_sync(0xffffffffu, g == k ? key : kFloatKeyNegInf);
+            if (lane == 0) atomicMax(p.best + (size_t)l * p.bestGroups + k, top);
+        }
+    };
+    int end = (l + 1) * p.cGroup - (j0 + c0);                   // group l's end in the chunk
+    if (end >= cn && cn == 32) {                                // one group
+        float m = v[0];
+#pragma unroll
+        for (int i = 1; i < 32; i++) m = fmaxf(m, v[i]);
+        put(m);
+    } else if (p.cGroup >= 32) {                                // two, or the tile's last columns
+        float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+            m0 = fmaxf(m0, i < end && i < cn ? v[i] : -INFINITY);
+            m1 = fmaxf(m1, i >= end && i < cn ? v[i] : -INFINITY);
+        }
+        put(m0);
+        if (end < cn) {
+            l++;
+            put(m1);
+        }
+    } else {
+        float m = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+            if (i >= cn) break;
+            m = fmaxf(m, v[i]);
+            if (i + 1 == end || i + 1 == cn) {
+                put(m);
+                m = -INFINITY;
+                l++;
+                end += p.cGroup;
+            }
+        }
+    }
+}
+
+// Half `half` of the accumulator's 32 lanes of this warp to C: lane = row;
+// columns go through the warp's buffer 32 at a time (TC_ROWS rows a time), so
+// that a store covers neighbouring columns.
+__device__ __forceinline__ void store_tile(const TcParams& p, uint32_t acc, float* stage,
+                                           const float* ad, int lane, int rowBase, int item,
+                                           int nValid, int half)
+{
+    const int rows = min(32, p.M - rowBase);
+    const float add = (lane < rows && p.nrm) ? p.nrm[item * p.sN + rowBase + lane] : 0.f;
+    float* cbase = p.C + item * p.sC + (size_t)rowBase * p.ldc;
+    const int j0 = item * p.colPerItem;
+    for (int c0 = 32 * half; c0 < nValid; c0 += 64) {
+        float v[32];
+        tmem_ld32(acc + (uint32_t)c0, v);
+        if (rows <= 0) continue;
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] = fmaf(p.alpha, v[i], add);
+        const int cn = min(32, nValid - c0);
+        if (p.best) chunk_best(p, v, cn, ad, lane, rowBase, rows, j0, c0);
+        size_t off = c0 + lane;
+        if (p.cGroup > 0) {
+            const int jj = j0 + c0 + lane, l = jj / p.cGroup;
+            off = (size_t)l * p.cGroupStride + (jj - l * p.cGroup);
+        }
+        float* dst = cbase + off;
+#pragma unroll
+        for (int h = 0; h < 32; h += TC_ROWS) {
+            if (lane / TC_ROWS == h / TC_ROWS)
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    *reinterpret_cast<float4*>(stage + (lane - h) * TC_PITCH + 4 * i) =
+                        make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            __syncwarp();
+            if (lane < cn) {
+                if (rows >= h + TC_ROWS) {
+                    float t[TC_ROWS];
+#pragma unroll
+                    for (int rr = 0; rr < TC_ROWS; rr++) t[rr] = stage[rr * TC_PITCH + lane];
+#pragma unroll
+                    for (int rr = 0; rr < TC_ROWS; rr++) dst[(long long)(h + rr) * p.ldc] = t[rr];
+                } else {
+                    for (int rr = 0; rr < rows - h; rr++)
+                        dst[(long long)(h + rr) * p.ldc] = stage[rr * TC_PITCH + lane];
+                }
+            }
+            __syncwarp();
+        }
+    }
 }
 
 template <int BK>
@@ -72,17 +210,18 @@ k_gemm_bf16x3(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ 
     const int aBytes = TC_M * BK * 2;                  // 16 KB (BK 64) or 8 KB (32)
     const int bBytes = p.ntile * BK * 2;               // ntile rows of 2 BK bytes
     const int stageBytes = 2 * aBytes + 2 * bBytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stageBytes);
+    float* outStage = reinterpret_cast<float*>(smem + p.stages * stageBytes);
+    float* norms = outStage + TC_EPI * TC_STAGE;                 // with best: [TC_EPI][32 TC_SEGS]
+    uint64_t* full =
+        reinterpret_cast<uint64_t*>(norms + (p.best ? TC_EPI * 32 * TC_SEGS : 0));
     uint64_t* empty = full + p.stages;
-    uint64_t* accum = empty + p.stages;
-    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(accum + 1);
+    uint64_t* accFull = empty + p.stages;              // [2]
+    uint64_t* accEmpty = accFull + 2;                  // [2]
+    uint64_t* drained = accEmpty + 2;                  // abort only: the issued MMAs are done
+    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(drained + 1);
     int* abortFlag = reinterpret_cast<int*>(tmemSlot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mtile = blockIdx.x, item = blockIdx.y;
-    const int aRow0 = item * p.aRowsPerItem + mtile * TC_M;
-    const int bRow0 = item * p.bRowsPerItem;
-    const int nValid = p.nTotal > 0 ? min(p.N, p.nTotal - item * p.N) : p.N;
     const int nkb = p.Kd / BK;
 
     if (threadIdx.x == 0) {
@@ -90,14 +229,18 @@ k_gemm_bf16x3(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ 
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
-        mbar_init(accum, 1);
+        for (int a = 0; a < 2; a++) {
+            mbar_init(accFull + a, 1);
+            mbar_init(accEmpty + a, TC_EPI);
+        }
+        mbar_init(drained, 1);
         *abortFlag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
+    if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmemSlot)),
-                     "r"(p.tmemCols)
+                     "r"(2 * p.tmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -105,118 +248,109 @@ k_gemm_bf16x3(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmemSlot;
+    // a wait that ran out anywhere in the CTA ends every role's loop
+    auto wait = [&](uint64_t* bar, int parity) {
+        if (mbar_wait(bar, parity, kWaitBudget) && *(volatile int*)abortFlag == 0) return true;
+        if (atomicExch(abortFlag, 1) == 0) atomicOr(p.flag, 4);
+        return false;
+    };
 
     int issuedTma = 0;      // K blocks whose copies were issued (producer)
     int issuedMma = 0;      // K blocks whose MMAs were issued (issuer)
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer
-        for (int kb = 0; kb < nkb; kb++) {
-            const int s = kb % p.stages;
-            const int round = kb / p.stages;
-            if (round > 0 && !mbar_wait(empty + s, (round - 1) & 1, kWaitBudget)) {
-                atomicOr(p.flag, 4);
-                *(volatile int*)abortFlag = 1;
-                break;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
+            const int item = t / p.mTiles;
+            const int aRow0 = item * p.aRowsPerItem + (t - item * p.mTiles) * TC_M;
+            const int bRow0 = item * p.bRowsPerItem;
+            for (int kb = 0; kb < nkb; kb++) {
+                const int s = issuedTma % p.stages, round = issuedTma / p.stages;
+                if (round > 0 && !wait(empty + s, (round - 1) & 1)) {
+                    ok = false;
+                    break;
+                }
+                uint8_t* st = smem + s * stageBytes;
+                mbar_expect_tx(full + s, stageBytes);
+                tma_load_2d(st, &tmAh, full + s, kb * BK, aRow0);
+                tma_load_2d(st + aBytes, &tmAl, full + s, kb * BK, aRow0);
+                tma_load_2d(st + 2 * aBytes, &tmBh, full + s, kb * BK, bRow0);
+                tma_load_2d(st + 2 * aBytes + bBytes, &tmBl, full + s, kb * BK, bRow0);
+                issuedTma++;
             }
-            if (*(volatile int*)abortFlag) break;
-            uint8_t* st = smem + s * stageBytes;
-            mbar_expect_tx(full + s, stageBytes);
-            tma_load_2d(st, &tmAh, full + s, kb * BK, aRow0);
-            tma_load_2d(st + aBytes, &tmAl, full + s, kb * BK, aRow0);
-            tma_load_2d(st + 2 * aBytes, &tmBh, full + s, kb * BK, bRow0);
-            tma_load_2d(st + 2 * aBytes + bBytes, &tmBl, full + s, kb * BK, bRow0);
-            issuedTma = kb + 1;
         }
     } else if (warp == 1 && lane == 0) {
         // ---------------- MMA issuer
         const uint32_t idesc = umma_idesc(TC_M, p.ntile);
-        for (int kb = 0; kb < nkb; kb++) {
-            const int s = kb % p.stages;
-            const int round = kb / p.stages;
-            if (!mbar_wait(full + s, round & 1, kWaitBudget)) {
-                atomicOr(p.flag, 4);
-                *(volatile int*)abortFlag = 1;
-                break;
-            }
-            if (*(volatile int*)abortFlag) break;
+        bool ok = true;
+        int i = 0;
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x, i++) {
+            const uint32_t acc = tmem + (i & 1) * p.tmemCols;
+            if (i >= 2 && !wait(accEmpty + (i & 1), ((i >> 1) - 1) & 1)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint8_t* st = smem + s * stageBytes;
-            const uint32_t ah = smem_u32(st), al = smem_u32(st + aBytes);
-            const uint32_t bh = smem_u32(st + 2 * aBytes), bl = smem_u32(st + 2 * aBytes + bBytes);
-#pragma unroll
-            for (int kk = 0; kk < BK / 16; kk++) {
-                const uint32_t off = kk * 32;      // 16 bf16 = 32 bytes along K
-                umma_bf16(tmem, desc<BK>(ah + off), desc<BK>(bh + off), idesc,
-                          (kb | kk) != 0);
-                umma_bf16(tmem, desc<BK>(ah + off), desc<BK>(bl + off), idesc, 1);
-                umma_bf16(tmem, desc<BK>(al + off), desc<BK>(bh + off), idesc, 1);
-            }
-            umma_commit(empty + s);        // stage free once these MMAs have read it
-            issuedMma = kb + 1;
-        }
-        umma_commit(accum);                // all issued MMAs complete -> epilogue
-    }
-    __syncthreads();
-    // ---------------- epilogue (all four warps)
-    bool ok = *(volatile int*)abortFlag == 0 && mbar_wait(accum, 0, kWaitBudget);
-    // block-uniform decision (the tcgen05.ld below is warp-collective)
-    ok = __syncthreads_and(ok) != 0;
-    if (!ok && threadIdx.x == 0) {
-        atomicOr(p.flag, 4);
-        *(volatile int*)abortFlag = 1;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const bool aborted = !ok;
-    if (!aborted) {
-        // The pipeline stages are free once the accumulator is complete: stage
-        // the warp's 32 rows there, then write every row with lanes over
-        // columns (coalesced).  Rows are padded by one float so both the
-        // column-wise fill and the row-wise drain are free of bank conflicts.
-        const int pitch = p.ntile + 1;
-        float* stage = reinterpret_cast<float*>(smem) + (size_t)warp * 32 * pitch;
-        const int rowBase = mtile * TC_M + warp * 32;
-        const bool rowOk = rowBase + lane < p.M;
-        const float add = (rowOk && p.nrm) ? p.nrm[item * p.sN + rowBase + lane] : 0.f;
-        for (int c0 = 0; c0 < p.ntile; c0 += 16) {
-            float v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-#pragma unroll
-            for (int i = 0; i < 16; i++) stage[lane * pitch + c0 + i] = fmaf(p.alpha, v[i], add);
-        }
-        __syncwarp();
-        float* cbase = p.C + item * p.sC;
-        for (int rr = 0; rr < 32; rr++) {
-            const int r = rowBase + rr;
-            if (r >= p.M) break;
-            for (int j = lane; j < nValid; j += 32) {
-                size_t off;
-                if (p.cGroup > 0) {
-                    const int jj = item * p.colPerItem + j;
-                    const int l = jj / p.cGroup;
-                    off = (size_t)l * p.cGroupStride + (size_t)r * p.ldc + (jj - l * p.cGroup);
-                } else {
-                    off = (size_t)r * p.ldc + j;
+            for (int kb = 0; kb < nkb; kb++) {
+                const int s = issuedMma % p.stages;
+                if (!wait(full + s, (issuedMma / p.stages) & 1)) {
+                    ok = false;
+                    break;
                 }
-                cbase[off] = stage[rr * pitch + j];
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint8_t* st = smem + s * stageBytes;
+                const uint32_t ah = smem_u32(st), al = smem_u32(st + aBytes);
+                const uint32_t bh = smem_u32(st + 2 * aBytes),
+                               bl = smem_u32(st + 2 * aBytes + bBytes);
+#pragma unroll
+                for (int kk = 0; kk < BK / 16; kk++) {
+                    const uint32_t off = kk * 32;      // 16 bf16 = 32 bytes along K
+                    umma_bf16(acc, desc<BK>(ah + off), desc<BK>(bh + off), idesc, (kb | kk) != 0);
+                    umma_bf16(acc, desc<BK>(ah + off), desc<BK>(bl + off), idesc, 1);
+                    umma_bf16(acc, desc<BK>(al + off), desc<BK>(bh + off), idesc, 1);
+                }
+                umma_commit(empty + s);    // stage free once these MMAs have read it
+                issuedMma++;
             }
+            if (ok) umma_commit(accFull + (i & 1));
+        }
+    } else if (warp >= 2) {
+        // ---------------- epilogue: tensor-memory lanes 32 (warp mod 4) ..
+        const int q = warp & 3;
+        int i = 0;
+        for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, i++) {
+            const int item = t / p.mTiles;
+            const int rowBase = (t - item * p.mTiles) * TC_M + q * 32;
+            const int nValid = p.nTotal > 0 ? min(p.N, p.nTotal - item * p.N) : p.N;
+            float* ad = norms + (warp - 2) * 32 * TC_SEGS;
+            if (p.best) load_norms(p, ad, lane, rowBase, item, nValid);
+            // one lane waits for the warp: the loads below are warp-collective
+            int ok = lane == 0 ? wait(accFull + (i & 1), (i >> 1) & 1) : 0;
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            store_tile(p, tmem + (i & 1) * p.tmemCols + ((uint32_t)(q * 32) << 16),
+                       outStage + (warp - 2) * TC_STAGE, ad, lane, rowBase, item, nValid,
+                       (warp - 2) >> 2);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(accEmpty + (i & 1));
         }
     }
-    // on an abort, let the copies this CTA issued land before leaving
-    if (aborted && warp == 0 && lane == 0) {
-        for (int kb = 0; kb < issuedTma; kb++) {
-            const int s = kb % p.stages;
-            mbar_wait(full + s, (kb / p.stages) & 1, kWaitBudget / 4);
+    __syncwarp();
+    __syncthreads();
+    if (*(volatile int*)abortFlag) {
+        // let the copies and the MMAs that this CTA issued finish before leaving
+        if (warp == 0 && lane == 0)
+            for (int kb = max(0, issuedTma - p.stages); kb < issuedTma; kb++)
+                mbar_wait(full + kb % p.stages, (kb / p.stages) & 1, kWaitBudget / 4);
+        if (warp == 1 && lane == 0 && issuedMma > 0) {
+            umma_commit(drained);
+            mbar_wait(drained, 0, kWaitBudget / 4);
         }
     }
-    // on an abort, the MMA issuer waits (bounded) for the MMAs it issued
-    if (aborted && warp == 1 && lane == 0 && issuedMma > 0)
-        mbar_wait(accum, 0, kWaitBudget / 4);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"(p.tmemCols)
+                     "r"(2 * p.tmemCols)
                      : "memory");
     }
 }
@@ -269,7 +403,7 @@ __device__ __forceinline__ void umma_commit_mc(uint64_t* bar, uint16_t mask)
 }
 
 template <int BK>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(128, 1)
 k_gemm_bf16x3_pair(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                    const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl,
                    const TcParams p)
@@ -444,7 +578,7 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
                                int bRowsPerItem, int nTotal, float* C, long long sC, int ldc,
                                const float* nrm, long long sN, float alpha, int* flag,
                                cudaStream_t st, int cGroup, long long cGroupStride, bool pair,
-                               int bk)
+                               int bk, const TileBest* best, bool besideProjections)
 {
     if (bk != 64 && bk != 32) return cudaErrorInvalidValue;
     if (N <= 0 || N > 256 || M <= 0 || items <= 0 || Kd <= 0 || Kd % bk)
@@ -466,13 +600,24 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
     p.ntile = (N + 15) / 16 * 16;
     p.tmemCols = 32;
     while (p.tmemCols < p.ntile) p.tmemCols <<= 1;
+    p.best = best ? best->key : nullptr;
+    if (best) {
+        if (pair || cGroup <= 0 || best->rows <= 0) return cudaErrorInvalidValue;
+        p.bestRows = best->rows;
+        p.bestGroups = best->groups;
+        p.bestNrm = best->nrm;
+        p.bestNs = best->nrmStride;
+    }
     const int stageBytes = 2 * TC_M * bk * 2 + 2 * p.ntile * bk * 2;
-    p.stages = (200 * 1024) / stageBytes;
+    // all of the shared memory; beside projections 131 KB (the 132 KB split of
+    // an SM's 228 KB with the CTA's own KB), at least two stages
+    const size_t extra = 1024 + 256 +
+                         sizeof(float) * TC_EPI * (TC_STAGE + (best ? 32 * TC_SEGS : 0));
+    p.stages = (int)(((besideProjections ? 131 : 227) * 1024 - extra) / stageBytes);
+    if (p.stages < 2) p.stages = (int)((227 * 1024 - extra) / stageBytes);
     const int maxStages = bk == 64 ? 4 : 6;
     if (p.stages > maxStages) p.stages = maxStages;
     if (p.stages < 2) return cudaErrorInvalidValue;
-    // the epilogue stages 128 rows of ntile + 1 floats in the pipeline buffers
-    if ((size_t)TC_M * (p.ntile + 1) * 4 > (size_t)p.stages * stageBytes) return cudaErrorInvalidValue;
     p.C = C;
     p.sC = sC;
     p.ldc = ldc;
@@ -487,9 +632,15 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
         !tc::make_map(&mBh, Bh, rowsB, Kd, p.ntile, bk, sw64) ||
         !tc::make_map(&mBl, Bl, rowsB, Kd, p.ntile, bk, sw64))
         return cudaErrorInvalidValue;
-    const size_t smem = 1024 + (size_t)p.stages * stageBytes + 256;
     const int mTiles = (M + TC_M - 1) / TC_M;
+    if ((long long)mTiles * items > 0x7fffffffLL) return cudaErrorInvalidValue;
+    p.mTiles = mTiles;
+    p.tiles = mTiles * items;
     if (pair && mTiles >= 2) {
+        // the epilogue stages 128 rows of ntile + 1 floats in the pipeline buffers
+        if ((size_t)TC_M * (p.ntile + 1) * 4 > (size_t)p.stages * stageBytes)
+            return cudaErrorInvalidValue;
+        const size_t smem = 1024 + (size_t)p.stages * stageBytes + 256;
         // CTA pairs on neighbouring row tiles (an odd count gets a tile of
         // rows past M, zero-filled by TMA and not stored); each loads half of
         // the B rows, multicast to both
@@ -504,7 +655,7 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)((mTiles + 1) / 2 * 2), (unsigned)items);
-        cfg.blockDim = dim3(TC_THREADS);
+        cfg.blockDim = dim3(128);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
@@ -516,13 +667,13 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
         cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, kern, mAh, mAl, hBh, hBl, p);
     }
+    const size_t smem = (size_t)p.stages * stageBytes + extra;
     void (*kern)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                  const TcParams) = bk == 64 ? k_gemm_bf16x3<64> : k_gemm_bf16x3<32>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid(mTiles, items);
-    kern<<<grid, TC_THREADS, smem, st>>>(mAh, mAl, mBh, mBl, p);
+    kern<<<std::min(p.tiles, 152), TC_THREADS, smem, st>>>(mAh, mAl, mBh, mBl, p);
     return cudaGetLastError();
 }
 
@@ -538,7 +689,7 @@ cudaError_t launch_gemm_nt_bf16x3(const float* A, long long sA, int lda, const f
         return cudaErrorInvalidValue;
     return launch_gemm_bf16x3(A, (long long)batch * M, B, (long long)batch * N, M, N, Kd, batch, M,
                               N, 0, C, sC, ldc, nrm, sN, alpha, flag, st, 0, 0, false,
-                              Kd % bk == 0 ? bk : 64);
+                              Kd % bk == 0 ? bk : 64, nullptr, true);
 }
 
 }  // namespace tg3
