@@ -30,6 +30,7 @@
 #include <mutex>
 #include <vector>
 
+#include "tg3_fft.cuh"
 #include "tg3_internal.cuh"
 
 namespace tg3 {
@@ -241,6 +242,381 @@ __global__ void k_acc_load(const float2* __restrict__ F, const float* __restrict
         acc[i] = make_float4(F[i].x, F[i].y, T[i], 0.f);
 }
 
+// ----------------------------------------------------------- own passes --
+// The 3-D reconstruction on grids whose side is in TG3_RECO_SIDES, as passes
+// over one half-complex array C [z][y][px], each line transformed on chip
+// (tg3_fft.cuh).  A balancing round:
+//   z: forward along z, W and C = T W updated, inverse along z;
+//   y: inverse;  x: inverse to two real rows, the kernel product, forward;
+//   y: forward.
+// C is zero and not looked at outside the sphere |k|^2 < r2max, so C keeps the
+// columns x < rmax only, the y passes read (inverse) or write (forward) the
+// rows inside the circle of their column, and the z pass visits those lines
+// only.  Bound by HBM: a round moves about 4 GB at 512^3 with rmax 240 and
+// takes 1.2 ms, where the library's six transform kernels and two passes
+// between them took 2.35 ms.
+struct Pass3 {
+    const float2* tw;        // the n-th roots of unity
+    float2* C;               // [n][n][px]
+    int nxr, px;             // columns in use, their pitch
+    long long r2max;
+};
+
+using fft::c64;
+
+template <int A, int B>
+__device__ __forceinline__ const float2* pass_roots(const Pass3& p, c64* buf)
+{
+    float2* tw = reinterpret_cast<float2*>(buf + fft::Shape<A, B>::floats2);
+    for (int k = threadIdx.x; k < A * B; k += blockDim.x) tw[k] = p.tw[k];
+    return tw;
+}
+
+// largest |y| with x0^2 + y^2 < r2max (x0 in use)
+__device__ __forceinline__ int rows_inside(long long r2max, int x0)
+{
+    const int q = (int)(r2max - 1 - (long long)x0 * x0);
+    int y = (int)sqrtf((float)q);
+    while ((long long)y * y > q) y--;
+    while ((long long)(y + 1) * (y + 1) <= q) y++;
+    return y;
+}
+
+__device__ __forceinline__ void copy16(float* dst, const float* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+
+__device__ __forceinline__ c64 load_c(const float2* p) { return *reinterpret_cast<const c64*>(p); }
+
+// CTA (8 columns, plane z): lines along y.
+template <int A, int B>
+__global__ void __launch_bounds__(fft::Shape<A, B>::threads, 384 / fft::Shape<A, B>::threads)
+k_reco_pass_y(const Pass3 p, int inverse, int planes)
+{
+    using S = fft::Shape<A, B>;
+    extern __shared__ __align__(16) c64 fsm[];
+    constexpr int n = S::n;
+    const int x0 = blockIdx.x * kFftLines, line = threadIdx.x % kFftLines, t = threadIdx.x / kFftLines;
+    const float2* tw = pass_roots<A, B>(p, fsm);
+    // planes < n: the central ones (coordinates -planes / 2 .. planes / 2 - 1)
+    const int z = blockIdx.y < planes / 2 ? blockIdx.y : blockIdx.y + n - planes;
+    float2* C = p.C + (size_t)z * n * p.px + x0 + line;
+    const int yr = rows_inside(p.r2max, x0);
+    c64 v[S::I1][A], o[S::I2][B];
+#pragma unroll
+    for (int i = 0; i < S::I1; i++)
+#pragma unroll
+        for (int r = 0; r < A; r++) {
+            const int y = t + i * S::TL + r * B;
+            v[i][r] = 0;
+            if (t + i * S::TL < B && (!inverse || y <= yr || n - y <= yr)) {
+                v[i][r] = load_c(C + (size_t)y * p.px);
+                if (inverse) v[i][r] = fft::swapped(v[i][r]);
+            }
+        }
+    __syncthreads();
+    fft::run<A, B, S::TL>(v, o, fsm, tw, t, line);
+#pragma unroll
+    for (int i = 0; i < S::I2; i++)
+#pragma unroll
+        for (int s = 0; s < B; s++) {
+            const int y = t + i * S::TL + s * A;
+            if (t + i * S::TL < A && (inverse || y <= yr || n - y <= yr))
+                *reinterpret_cast<c64*>(C + (size_t)y * p.px) =
+                    inverse ? fft::swapped(o[i][s]) : o[i][s];
+        }
+}
+
+// CTA (8 columns, row y inside their circle): lines along z.  Mode 0: T from
+// the accumulator and the FSC (rfsc [nFsc + 1]: 1 / f of a shell, the last for
+// shells past its end), W = 1, C = T; 1: a round's update; 2: C = F W; 3: C = F /
+// T, no grid correction.  Then the inverse along z.
+template <int A, int B>
+__global__ void __launch_bounds__(fft::Shape<A, B>::threads, 384 / fft::Shape<A, B>::threads)
+k_reco_pass_z(const Pass3 p, int mode, const float4* __restrict__ acc,
+              const double* __restrict__ rfsc, int nFsc, int pf, float* __restrict__ T,
+              float* __restrict__ W, unsigned* __restrict__ diffBits)
+{
+    using S = fft::Shape<A, B>;
+    extern __shared__ __align__(16) c64 fsm[];
+    constexpr int n = S::n;
+    const int x0 = blockIdx.x * kFftLines, line = threadIdx.x % kFftLines, t = threadIdx.x / kFftLines;
+    const int rmax = rows_inside(p.r2max, 0);
+    const int yc = (int)blockIdx.y - rmax;
+    if ((long long)x0 * x0 + (long long)yc * yc >= p.r2max) return;
+    const float2* tw = pass_roots<A, B>(p, fsm);
+    const int y = yc < 0 ? yc + n : yc, x = x0 + line;
+    const size_t at0 = (size_t)y * p.px + x, plane = (size_t)n * p.px;
+    const int xy = x * x + yc * yc, r2 = (int)p.r2max;
+    const int xa = min(x, n / 2);
+    c64 v[S::I1][A], o[S::I2][B];
+    // a round's W and T of the inside of the line, copied behind the first
+    // transform
+    float* sW = reinterpret_cast<float*>(fsm + S::smem / sizeof(c64));
+    float* sT = sW + n * kFftLines;
+    if (mode == 1) {
+        const int zr = rows_inside(p.r2max - yc * yc, x0);
+        for (int i = threadIdx.x; i < n * 2; i += S::threads) {
+            const int z = i >> 1, e = 4 * (i & 1);
+            if (z > zr && n - z > zr) continue;
+            const size_t g = z * plane + (size_t)y * p.px + x0 + e;
+            copy16(sW + z * kFftLines + e, W + g);
+            copy16(sT + z * kFftLines + e, T + g);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < S::I1; i++)
+#pragma unroll
+            for (int r = 0; r < A; r++) {
+                const int z = t + i * S::TL + r * B;
+                v[i][r] = t + i * S::TL < B ? load_c(p.C + z * plane + at0) : 0;
+            }
+        __syncthreads();
+        fft::run<A, B, S::TL>(v, o, fsm, tw, t, line);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    float dmax = 0.f;
+    // points outside the sphere read an inside one's neighbourhood of their
+    // line (z = 0 lies inside), so that a group's loads go out together
+    constexpr int G = 8;
+#pragma unroll
+    for (int i = 0; i < S::I2; i++)
+#pragma unroll
+        for (int s0 = 0; s0 < B; s0 += G) {
+            float4 f[G];
+            float w[G], tt[G];
+            bool in[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const int z = t + i * S::TL + (s0 + g) * A;
+                const int zc = z < n / 2 ? z : z - n;
+                in[g] = s0 + g < B && t + i * S::TL < A && xy + zc * zc < r2;
+                const int zl = in[g] ? z : 0;
+                const size_t at = zl * plane + at0;
+                if (mode == 1) {
+                    w[g] = sW[zl * kFftLines + line];
+                    tt[g] = sT[zl * kFftLines + line];
+                }
+                if (mode == 2) w[g] = W[at];
+                if (mode != 1) f[g] = acc[((size_t)zl * n + y) * (n / 2 + 1) + xa];
+            }
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                if (s0 + g >= B) break;
+                const int z = t + i * S::TL + (s0 + g) * A;
+                const int zc = z < n / 2 ? z : z - n;
+                const int q = xy + zc * zc;
+                const size_t at = z * plane + at0;
+                float2 c = make_float2(0.f, 0.f);
+                if (mode == 1) {
+                    const float2 u = fft::unpack(o[i][s0 + g]);
+                    const float m = sqrtf(u.x * u.x + u.y * u.y);
+                    const float wn = w[g] / fmaxf(m, 1e-6f);
+                    if (in[g]) {
+                        W[at] = wn;
+                        dmax = fmaxf(dmax, fabsf(m - 1.f));
+                        c.x = tt[g] * wn;
+                    }
+                } else if (in[g]) {
+                    float tf = 0.f;
+                    if (mode != 2) {
+                        double d = f[g].z;
+                        if (rfsc && q >= 25 * pf * pf)
+                            d *= rfsc[min((int)rintf(sqrtf((float)q)) / pf, nFsc)];
+                        tf = (float)fmax(d, 1e-25);
+                    }
+                    if (mode == 0) {
+                        c.x = tf;
+                        T[at] = tf;
+                        W[at] = 1.f;
+                    } else {
+                        const float wn = mode == 2 ? w[g] : 1.f / fmaxf(tf, 1e-6f);
+                        c = make_float2(f[g].x * wn, f[g].y * wn);
+                    }
+                }
+                o[i][s0 + g] = fft::pack(c.y, c.x);   // exchanged: the inverse transform
+            }
+        }
+    fft::run<B, A, S::TL>(o, v, fsm, tw, t, line);
+#pragma unroll
+    for (int i = 0; i < S::I1; i++)
+#pragma unroll
+        for (int r = 0; r < A; r++)
+            if (t + i * S::TL < B)
+                *reinterpret_cast<c64*>(p.C + (t + i * S::TL + r * B) * plane + at0) =
+                    fft::swapped(v[i][r]);
+    if (mode == 1) {
+        for (int k = 16; k; k >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, k));
+        if ((threadIdx.x & 31) == 0) atomicMax(diffBits, __float_as_uint(dmax));
+    }
+}
+
+// CTA (8 pairs of rows, plane z): pair l holds the rows y = l and n - l (0 and
+// n / 2 for l = 0), whose points share the kernel's argument, as the real and
+// the imaginary part of one complex line.  With out: the real rows' central N
+// points over tab to out [N][N][N]; else times the kernel and forward again.
+// The kernel comes as a grid over one octant, kgrid [z][l / 8][x][8]: looked up
+// in tab (over the integer squared radius) every point costs a sector of L2,
+// four times the bytes of C; tab serves the row n / 2 of the pair 0.
+template <int A, int B>
+__global__ void __launch_bounds__(fft::Shape<A, B>::threads, 384 / fft::Shape<A, B>::threads)
+k_reco_pass_x(const Pass3 p, const float* __restrict__ tab, const float* __restrict__ kgrid, int N,
+              float* __restrict__ out)
+{
+    using S = fft::Shape<A, B>;
+    extern __shared__ __align__(16) c64 fsm[];
+    constexpr int n = S::n, h = n / 2;
+    const int line = threadIdx.x % kFftLines, t = threadIdx.x / kFftLines;
+    const int l = blockIdx.x * kFftLines + line;
+    const float2* tw = pass_roots<A, B>(p, fsm);
+    const int z = !out || blockIdx.y < N / 2 ? blockIdx.y : blockIdx.y + n - N;
+    const int zc = z < h ? z : z - n;
+    float2* C = p.C + (size_t)z * n * p.px;
+    const int ll = min(l, h - 1);               // lines past the last pair are not stored
+    // the 16 rows, copied whole and read in both directions (from global memory
+    // every access would touch eight rows); their pitch spreads eight rows
+    // over the banks
+    const int pitch = (p.px + 15) / 16 * 16 + 2;
+    float2* rows = reinterpret_cast<float2*>(fsm + S::smem / sizeof(c64));
+    for (int i = threadIdx.x; i < 2 * kFftLines * (p.px / 2); i += S::threads) {
+        const int r = i / (p.px / 2), e = 2 * (i % (p.px / 2));
+        const int q = min(blockIdx.x * kFftLines + r % kFftLines, h - 1);
+        const int y = r < kFftLines ? q : (q ? n - q : h);
+        copy16(reinterpret_cast<float*>(rows + r * pitch + e),
+               reinterpret_cast<const float*>(C + (size_t)y * p.px + e));
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const float2* row0 = rows + line * pitch;
+    const float2* row1 = row0 + kFftLines * pitch;
+    c64 v[S::I1][A], o[S::I2][B];
+#pragma unroll
+    for (int i = 0; i < S::I1; i++)
+#pragma unroll
+        for (int r = 0; r < A; r++) {
+            const int k = t + i * S::TL + r * B;
+            const int m = k < p.nxr ? k : n - k;     // the stored column, or the mirrored one
+            const bool in = t + i * S::TL < B && m < p.nxr;
+            const int ml = min(m, p.nxr - 1);
+            const float2 a = row0[ml], b = row1[ml];
+            // a + i b, real and imaginary part exchanged: the inverse transform
+            const float2 u = k == 0      ? make_float2(b.x, a.x)
+                             : k < p.nxr ? make_float2(a.y + b.x, a.x - b.y)
+                                         : make_float2(b.x - a.y, a.x + b.y);
+            v[i][r] = in ? fft::pack(u.x, u.y) : 0;
+        }
+    fft::run<A, B, S::TL>(v, o, fsm, tw, t, line);
+    if (out) {
+#pragma unroll
+        for (int i = 0; i < S::I2; i++)
+#pragma unroll
+            for (int s = 0; s < B; s++) {
+                const int x = t + i * S::TL + s * A;
+                const int xc = x < h ? x : x - n, y1 = l ? -l : -h;
+                if (t + i * S::TL >= A || l >= h || xc < -N / 2 || xc >= N / 2) continue;
+                const float2 u = fft::unpack(o[i][s]);        // (row 1, row 0)
+                const size_t at = ((size_t)(zc + N / 2) * N + N / 2) * N + xc + N / 2;
+                if (l < N / 2) out[at + (long long)l * N] = u.y / tab[xc * xc + l * l + zc * zc];
+                if (y1 >= -N / 2)
+                    out[at + (long long)y1 * N] = u.x / tab[xc * xc + y1 * y1 + zc * zc];
+            }
+        return;
+    }
+    const int c = zc * zc + ll * ll;
+    const float* kg = kgrid + ((size_t)abs(zc) * gridDim.x + blockIdx.x) * ((h + 1) * kFftLines) + line;
+#pragma unroll
+    for (int i = 0; i < S::I2; i++) {
+        float kv[B];
+#pragma unroll
+        for (int s = 0; s < B; s++) {
+            const int x = min(t + i * S::TL, A - 1) + s * A;
+            const int xc = x <= h ? x : n - x;
+            kv[s] = __ldg(kg + xc * kFftLines);
+        }
+#pragma unroll
+        for (int s = 0; s < B; s++) {
+            const int x = min(t + i * S::TL, A - 1) + s * A;
+            const int xc = x <= h ? x : n - x;
+            const float k1 = ll ? kv[s] : __ldg(tab + xc * xc + c + h * h);
+            const float2 u = fft::unpack(o[i][s]);            // (row 1, row 0)
+            o[i][s] = fft::pack(u.y * kv[s], u.x * k1);
+        }
+    }
+    fft::run<B, A, S::TL>(o, v, fsm, tw, t, line);
+    // the two rows' spectra from the line's at k and n - k, a warp along a row
+    constexpr int lp = n + 2;
+#pragma unroll
+    for (int i = 0; i < S::I1; i++)
+#pragma unroll
+        for (int r = 0; r < A; r++)
+            if (t + i * S::TL < B) fsm[line * lp + t + i * S::TL + r * B] = v[i][r];
+    __syncthreads();
+    for (int i = threadIdx.x; i < kFftLines * p.px; i += S::threads) {
+        const int q = i / p.px, k = i % p.px, y = blockIdx.x * kFftLines + q;
+        if (y >= h || k >= p.nxr) continue;
+        const float2 a = fft::unpack(fsm[q * lp + k]), b = fft::unpack(fsm[q * lp + (k ? n - k : 0)]);
+        C[(size_t)y * p.px + k] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
+        C[(size_t)(y ? n - y : h) * p.px + k] = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
+    }
+}
+
+// kgrid [z][lt][x][8] = tab[x^2 + l^2 + z^2] for z, x <= h, l = 8 lt + lane
+__global__ void k_reco_kernel_grid(const float* __restrict__ tab, int h, int lt,
+                                   float* __restrict__ kgrid)
+{
+    const size_t total = (size_t)(h + 1) * lt * (h + 1) * kFftLines;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
+         i += (size_t)gridDim.x * blockDim.x) {
+        const unsigned u = (unsigned)(i / kFftLines);
+        const int x = (int)(u % (h + 1)), w = (int)(u / (h + 1));
+        const int l = min(w % lt * kFftLines + (int)(i % kFftLines), h), z = w / lt;
+        kgrid[i] = tab[x * x + l * l + z * z];
+    }
+}
+
+// sides with their two factors (the larger first)
+#define TG3_RECO_SIDES(X)                                                                        \
+    X(12, 8) X(16, 8) X(12, 12) X(16, 10) X(15, 12) X(16, 12) X(18, 12) X(16, 15) X(16, 16)      \
+        X(18, 16) X(20, 16) X(20, 18) X(24, 16) X(20, 20) X(24, 18) X(24, 20) X(32, 16)
+
+struct PassKernels {
+    void (*y)(Pass3, int, int);
+    void (*z)(Pass3, int, const float4*, const double*, int, int, float*, float*, unsigned*);
+    void (*x)(Pass3, const float*, const float*, int, float*);
+    int threads;
+    size_t smem;
+};
+
+bool pass_kernels(int n, PassKernels* k)
+{
+#define X(a, b)                                                                                    \
+    if (n == a * b) {                                                                              \
+        *k = {k_reco_pass_y<a, b>, k_reco_pass_z<a, b>, k_reco_pass_x<a, b>,                       \
+              fft::Shape<a, b>::threads, fft::Shape<a, b>::smem};                                  \
+        return true;                                                                               \
+    }
+    TG3_RECO_SIDES(X)
+#undef X
+    return false;
+}
+
+// 1 / f of every shell of the FSC, f clamped and joined as in k_reco_init
+__global__ void k_reco_rfsc(const double* __restrict__ fsc, int nFsc, int joinHalf,
+                            double* __restrict__ rfsc)
+{
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u <= nFsc; u += gridDim.x * blockDim.x) {
+        double f = u < nFsc ? fsc[u] : 0.0;
+        f = fmax(1e-3, fmin(1.0 - 1e-3, f));
+        if (joinHalf) f = sqrt(2.0 * f / (1.0 + f));
+        rfsc[u] = 1.0 / f;
+    }
+}
+
 struct Plan3 {
     tg3_ctx* c;
     int vdim, nz, type;
@@ -404,6 +780,107 @@ extern "C" int tg3_ctx_insert_load_d(tg3_ctx* c, const float* F, const float* T)
 
 namespace {
 
+// The stopping rule of the balancing rounds: round m's largest ||C| - 1| read
+// back and compared.
+struct Balance {
+    float diff = 3.4e38f;
+    int noDecrease = 0;
+    bool done(int m, float d)
+    {
+        noDecrease = d > diff * 0.95f ? noDecrease + 1 : 0;
+        diff = d;
+        return d < 1e-2f || (m >= 10 && noDecrease == 2);
+    }
+};
+
+int read_diff(tg3_ctx* c, const unsigned* dBits, float* d)
+{
+    unsigned bits = 0;
+    TG3_CUDA(cudaMemcpyAsync(&bits, dBits, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    TG3_CUDA(cudaStreamSynchronize(c->stream));
+    std::memcpy(d, &bits, sizeof(float));
+    return TG3_OK;
+}
+
+// 3-D reconstruction by the passes above.
+int reconstruct_passes(tg3_ctx* c, const PassKernels& k, const float4* acc, int n, int pf,
+                       const double* fsc, int nFsc, int joinHalf, int maxRadius, int gridCorr,
+                       int kernel, float a, float alpha, float* vol, int* rounds)
+{
+    int st = TG3_OK;
+    const int N = n / pf, rmax = maxRadius * pf;
+    Pass3 p;
+    p.nxr = rmax;
+    p.px = (rmax + kFftLines - 1) / kFftLines * kFftLines;
+    p.r2max = (long long)rmax * rmax;
+    const size_t cells = (size_t)n * n * p.px;
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const int nqPad = 3 * (n / 2) * (n / 2) + 1, nqBox = 3 * (N / 2) * (N / 2) + 1;
+    const size_t oT = 0, oW = up(4 * cells), oC = oW + up(4 * cells), oD = oC + up(8 * cells),
+                 oK = oD + 256, oE = oK + up(4 * (size_t)nqPad), oR = oE + up(4 * (size_t)nqBox),
+                 oF = oR + up(8 * (size_t)n), oG = oF + up(8 * (size_t)(nFsc + 1));
+    const int h = n / 2, lt = (h + kFftLines - 1) / kFftLines;
+    const size_t total =
+        oG + (gridCorr ? up(4 * (size_t)(h + 1) * lt * (h + 1) * kFftLines) : 256);
+    char* b = (char*)ws_get(c, WS_RECO, total, &st);
+    if (!b) return st;
+    float* T = (float*)(b + oT);
+    float* W = (float*)(b + oW);
+    p.C = (float2*)(b + oC);
+    unsigned* dBits = (unsigned*)(b + oD);
+    float* tabK = (float*)(b + oK);
+    float* tabE = (float*)(b + oE);
+    p.tw = (float2*)(b + oR);
+    double* rfsc = fsc ? (double*)(b + oF) : nullptr;
+    float* kgrid = (float*)(b + oG);
+    cudaStream_t s = c->stream;
+    const size_t smemZ = k.smem + 2 * sizeof(float) * (size_t)n * kFftLines;
+    const size_t smemX = k.smem + sizeof(float2) * 2 * kFftLines * ((p.px + 15) / 16 * 16 + 2);
+    TG3_CUDA(cudaFuncSetAttribute(k.y, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
+    TG3_CUDA(cudaFuncSetAttribute(k.x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemX));
+    TG3_CUDA(cudaFuncSetAttribute(k.z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemZ));
+    const double i0a = bessel_i0(alpha), cellsD = (double)n * n * n;
+    const double invNf = gridCorr ? 1.0 / mkb_rl(0.0, a, alpha, i0a) : 0.0;
+    fft::k_roots<<<(n + 127) / 128, 128, 0, s>>>(const_cast<float2*>(p.tw), n);
+    if (gridCorr) {
+        k_radial_table<<<(nqPad + 255) / 256, 256, 0, s>>>(tabK, nqPad, (double)N * pf, 1, a, alpha,
+                                                            i0a, invNf / cellsD, 1.0 / 100000);
+        k_reco_kernel_grid<<<152 * 8, 256, 0, s>>>(tabK, h, lt, kgrid);
+    }
+    if (rfsc) k_reco_rfsc<<<(nFsc + 128) / 128, 128, 0, s>>>(fsc, nFsc, joinHalf, rfsc);
+    const int xt = p.px / kFftLines;
+    const dim3 gz(xt, 2 * rmax - 1), gy(xt, n), gx(lt, n);
+    if (gridCorr)
+        k.z<<<gz, k.threads, smemZ, s>>>(p, 0, acc, rfsc, nFsc, pf, T, W, nullptr);
+    TG3_LAUNCH_CHECK("reconstruction set-up");
+    Balance bal;
+    int m = 0;
+    for (m = 0; gridCorr && m < 30; m++) {
+        k.y<<<gy, k.threads, k.smem, s>>>(p, 1, n);
+        k.x<<<gx, k.threads, smemX, s>>>(p, tabK, kgrid, N, nullptr);
+        k.y<<<gy, k.threads, k.smem, s>>>(p, 0, n);
+        TG3_CUDA(cudaMemsetAsync(dBits, 0, sizeof(unsigned), s));
+        k.z<<<gz, k.threads, smemZ, s>>>(p, 1, nullptr, nullptr, 0, pf, T, W, dBits);
+        TG3_LAUNCH_CHECK("balancing round");
+        float d = 0.f;
+        if ((st = read_diff(c, dBits, &d))) return st;
+        if (bal.done(m, d)) break;
+    }
+    if (rounds) *rounds = gridCorr ? std::min(m + 1, 30) : 0;
+    const int mkb = kernel == TG3_KERNEL_MKB;
+    const double nf = mkb ? mkb_rl(0.0, (double)a * pf, alpha, i0a) : 1.0;
+    k_radial_table<<<(nqBox + 255) / 256, 256, 0, s>>>(tabE, nqBox, (double)pf * N, mkb,
+                                                        (double)a * pf, alpha, i0a, cellsD / nf, 0.0);
+    if (gridCorr)
+        k.z<<<gz, k.threads, smemZ, s>>>(p, 2, acc, nullptr, 0, pf, T, W, nullptr);
+    else
+        k.z<<<gz, k.threads, smemZ, s>>>(p, 3, acc, rfsc, nFsc, pf, T, W, nullptr);
+    k.y<<<dim3(xt, N), k.threads, k.smem, s>>>(p, 1, N);
+    k.x<<<dim3(gx.x, N), k.threads, smemX, s>>>(p, tabE, nullptr, N, vol);
+    TG3_LAUNCH_CHECK("map from F W");
+    return TG3_OK;
+}
+
 // The reconstruction chain on an accumulator acc of vdim x vdim x (vdim/2+1)
 // cells (nz = vdim, 3-D) or vdim x (vdim/2+1) (nz = 1, 2-D), into out: the
 // central N^3 or N^2 of the padded real-space result, N = vdim / pf.
@@ -413,6 +890,13 @@ int reconstruct_core(tg3_ctx* c, const float4* acc, int vdim, int nz, int pf, co
 {
     int st = TG3_OK;
     const int N = vdim / pf;
+    // 3-D grids of the listed sides: own transforms fused with the rounds' other
+    // passes (512^3, 19 rounds: 48 -> 25 ms); other sides and the
+    // single-plane grids of a 2-D class by the library's
+    PassKernels own;
+    if (nz > 1 && N * pf == vdim && N % 2 == 0 && pass_kernels(vdim, &own))
+        return reconstruct_passes(c, own, acc, vdim, pf, fsc, nFsc, joinHalf, maxRadius, gridCorr,
+                                  kernel, a, alpha, vol, rounds);
     const double cells = nz > 1 ? (double)vdim * vdim * vdim : (double)vdim * vdim;
     const size_t nh = (size_t)nz * vdim * (vdim / 2 + 1), nr = (size_t)nz * vdim * vdim;
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
@@ -446,8 +930,7 @@ int reconstruct_core(tg3_ctx* c, const float4* acc, int vdim, int nz, int pf, co
         k_radial_table<<<(nqPad + 255) / 256, 256, 0, s>>>(tabK, nqPad, (double)N * pf, 1, a, alpha,
                                                             i0a, invNf / cells, 1.0 / 100000);
         TG3_LAUNCH_CHECK("balancing kernel table");
-        float diff = 3.4e38f, prev;
-        int noDecrease = 0;
+        Balance bal;
         k_reco_tw<<<G, 256, 0, s>>>(T, W, nh, C);
         TG3_LAUNCH_CHECK("balancing C = T W");
         for (m = 0; m < 30; m++) {
@@ -460,13 +943,9 @@ int reconstruct_core(tg3_ctx* c, const float4* acc, int vdim, int nz, int pf, co
             TG3_CUDA(cudaMemsetAsync(dBits, 0, sizeof(unsigned), s));
             k_reco_update<<<G, 256, 0, s>>>(C, T, vdim, nz, r2max, W, dBits);
             TG3_LAUNCH_CHECK("balancing update");
-            unsigned bits = 0;
-            TG3_CUDA(cudaMemcpyAsync(&bits, dBits, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-            TG3_CUDA(cudaStreamSynchronize(s));
-            prev = diff;
-            std::memcpy(&diff, &bits, sizeof(float));
-            noDecrease = diff > prev * 0.95f ? noDecrease + 1 : 0;
-            if (diff < 1e-2f || (m >= 10 && noDecrease == 2)) break;
+            float d = 0.f;
+            if ((st = read_diff(c, dBits, &d))) return st;
+            if (bal.done(m, d)) break;
         }
     } else {
         k_reco_w_from_t<<<G, 256, 0, s>>>(T, vdim, nz, r2max, W);
