@@ -32,9 +32,25 @@ def _half(vdim, rng):
     (60, 3, 25, False, "mkb"), (96, 2, 47, False, "mkb"), (54, 4, 20, False, "mkb"),
     (50, 2, 20, True, "mkb")])
 def test_sides(N, pf, max_r, grid, kernel):
-    rng = np.random.default_rng(N + max_r)
-    vdim = N * pf
+    F, T = _half(N * pf, np.random.default_rng(N + max_r))
+    _check(N, pf, max_r, grid, kernel, F, T)
+
+
+@pytest.mark.parametrize("N,grid", [(48, True), (64, True), (64, False), (72, True)])
+def test_unpaired_plane(N, grid):
+    """The column x = 0 as insertion leaves it: the writes to (0, y, z) and to
+    (0, -y, -z) come from different pixels, so the two are not conjugates.  The
+    real transform along x takes the real part of that column's sums."""
+    vdim = 2 * N
+    rng = np.random.default_rng(N)
     F, T = _half(vdim, rng)
+    F[:, :, 0] += 0.3 * (rng.standard_normal((vdim, vdim)) + 1j * rng.standard_normal((vdim, vdim)))
+    T[:, :, 0] *= rng.uniform(0.5, 1.5, (vdim, vdim))
+    _check(N, 2, N // 2 - 3, grid, "mkb", F, T)
+
+
+def _check(N, pf, max_r, grid, kernel, F, T):
+    vdim = N * pf
     fsc = np.clip(1.05 - np.arange(N // 2 + 1) / (N / 2), 0, 1)
     ctx = tg3.Context(0)
     try:
