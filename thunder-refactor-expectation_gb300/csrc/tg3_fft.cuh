@@ -14,7 +14,7 @@
 // transform of the points with real and imaginary part exchanged, exchanged
 // back (unnormalised, as the forward one).
 //
-// The small transforms are unrolled from radix 2, 3, 4, 5 and 8 with constant
+// The small transforms are unrolled from radix 2, 3, 4, 5 and (by their definition) 7, 11, 13 with constant
 // twiddles; the twiddles between the steps come from one table of the n-th
 // roots of unity (each rounded from an accurate sine and cosine), so the error
 // is that of the additions.  Additions work on (re, im) pairs.  A CTA has
@@ -151,6 +151,20 @@ constexpr int first_factor(int r)
 template <int R>
 __device__ __forceinline__ void dft(c64* v);
 
+// cosines and sines of 2 pi k / R
+template <int R>
+struct Circle {
+    float c[R] = {}, s[R] = {};
+    constexpr Circle()
+    {
+        for (int k = 0; k < R; k++) {
+            const Root w = root(k, R);
+            c[k] = (float)w.c;
+            s[k] = (float)w.s;
+        }
+    }
+};
+
 template <int R, int P, int Q, int I>
 __device__ __forceinline__ void twiddle_all(c64* u)
 {
@@ -196,6 +210,30 @@ __device__ __forceinline__ void dft(c64* v)
         v[4] = sub(m1, t1);
         v[2] = add(m2, t2);
         v[3] = sub(m2, t2);
+    } else if constexpr (R == 7 || R == 11 || R == 13) {
+        // X[k], X[R - k] = v[0] + sum_j (v[j] + v[R - j]) cos(2 pi j k / R)
+        //                  -+ i (v[j] - v[R - j]) sin(2 pi j k / R)
+        constexpr Circle<R> w;
+        constexpr int H = R / 2;
+        c64 a[H], b[H], sum = v[0];
+#pragma unroll
+        for (int j = 1; j <= H; j++) {
+            a[j - 1] = add(v[j], v[R - j]);
+            b[j - 1] = rot(sub(v[j], v[R - j]));
+            sum = add(sum, a[j - 1]);
+        }
+#pragma unroll
+        for (int k = 1; k <= H; k++) {
+            c64 m = v[0], t = scale(b[0], w.s[k]);
+#pragma unroll
+            for (int j = 1; j <= H; j++) {
+                m = mad(a[j - 1], pack(w.c[j * k % R], w.c[j * k % R]), m);
+                if (j > 1) t = mad(b[j - 1], pack(w.s[j * k % R], w.s[j * k % R]), t);
+            }
+            v[k] = add(m, t);
+            v[R - k] = sub(m, t);
+        }
+        v[0] = sum;
     } else {
         // x[q + Q p]: transforms of P over p, twiddles, transforms of Q over q
         constexpr int P = first_factor(R), Q = R / P;

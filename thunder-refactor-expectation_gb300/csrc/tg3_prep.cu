@@ -24,10 +24,13 @@
 #include <mutex>
 #include <vector>
 
+#include "tg3_fft.cuh"
 #include "tg3_internal.cuh"
 
 namespace tg3 {
 namespace {
+
+constexpr size_t kSmemCta = 227 * 1024, kSmemSm = 228 * 1024;   // dynamic of a CTA; of an SM
 
 __device__ double prep_block_sum(double v, double* scratch)
 {
@@ -45,104 +48,473 @@ __device__ double prep_block_sum(double v, double* scratch)
     return scratch[0];
 }
 
-// Per-image background statistics: stats[l] = (m, s, sN), sN the background
-// standard deviation of (x - m) / s about 0.  One pass: a warp per row, lanes
-// over columns; each lane sums its pixels of a row about a pivot (the
-// corner pixel, always background) in FP32 and adds the row's partial sums
-// to FP64 totals.  Background: i^2 + j^2 > r^2, i.e. > floor(r^2) in
-// integers.  CTA per image.
-__global__ void __launch_bounds__(256)
-k_bg_stats(const float* __restrict__ img, int N, long long bgAbove, double* __restrict__ st)
+// The soft mask as a function of the integer squared radius q = i^2 + j^2: 1 for
+// q <= qIn, tab[q - qIn] up to qOut, 0 beyond.
+struct SoftMask {
+    const float* tab;        // [qOut - qIn + 1], tab[0] = 1
+    int qIn, qOut;
+};
+
+// (x - m) f as (x - high part of m) f - (low part of m) f: the mean rounded to
+// FP32 would shift every pixel alike, which the lowest frequencies add up.
+struct Scaling {
+    float m, f, c;
+};
+
+__device__ __forceinline__ float scaled(const Scaling& a, float x) { return fmaf(x - a.m, a.f, a.c); }
+
+__device__ __forceinline__ float masked(float v, int q, const SoftMask& k, const float* tab)
 {
-    __shared__ double red[32];
+    const float w = tab[min(max(q - k.qIn, 0), k.qOut - k.qIn)];
+    return q > k.qOut ? 0.f : v * w;
+}
+
+// Per-image background statistics: st[l] = (m, s, sN, 1 / s), sN the background
+// standard deviation of (x - m) / s about 0.  One pass over the background's
+// pixels only, i^2 + j^2 > bgAbove = floor(r^2) in integers: a warp takes four
+// rows at a time, lanes over what lies left and right of the circle, eight
+// loads in flight; a lane sums eight pixels about a pivot (the corner pixel,
+// always background) in FP32 and adds that to totals held as a pair of FP32
+// (the sum and what its roundings lost, 48 bits together), which become FP64 at
+// the end: FP64 sums on the way, two lanes a clock, took most of the time.
+// Lanes past a row's end read the pivot, which adds nothing.  CTA per image;
+// 1,024 images of 256^2: 52 us (a load at a time and FP64 sums: 124).
+// The call's tables come along, spread over the CTAs: the soft mask's edge, w =
+// 1 - (0.5 - 0.5 cos((u - r) / ew pi)); the transform's twiddles w_N^(r j)
+// [A][B]; and where the pixels lie in the transform's columns.
+struct PrepTables {
+    float* mask;
+    int qIn, nMask;          // entries
+    float r, ew;
+    float2* tw;
+    int A, B;                // 0: no twiddles, no slots
+    int* slot;               // [K] (CTA of the image << 20) + place
+    const int *iCol, *iRow;
+    int K, cols, maxCol, W;
+};
+
+// a total and the part its roundings lost (Knuth's two-sum)
+struct Total {
+    float s, lost;
+    __device__ __forceinline__ void add(float v)
+    {
+        const float t = s + v, b = t - s;
+        lost += (s - (t - b)) + (v - b);
+        s = t;
+    }
+    __device__ __forceinline__ double value() const
+    {
+        return isinf(s) ? (double)s : (double)s + lost;
+    }
+    __device__ __forceinline__ void warp_sum()
+    {
+        for (int o = 16; o; o >>= 1) {
+            const float v = __shfl_xor_sync(0xffffffffu, s, o);
+            lost += __shfl_xor_sync(0xffffffffu, lost, o);
+            add(v);
+        }
+    }
+};
+
+__global__ void __launch_bounds__(256)
+k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double* __restrict__ st,
+           float* __restrict__ st32, const PrepTables t)
+{
+    extern __shared__ int2 rows[];               // [N rounded up to 4] (left, right) of the circle
+    __shared__ Total part[2][8];
     const size_t l = blockIdx.x;
+    if (threadIdx.x < 32)
+        for (int e = blockIdx.x * 32 + threadIdx.x; e < t.A * t.B; e += gridDim.x * 32) {
+            double s, c;
+            sincospi(-2.0 * (e / t.B * (e % t.B)) / (t.A * t.B), &s, &c);
+            t.tw[e] = make_float2((float)c, (float)s);
+        }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < max(t.nMask, t.K);
+         i += gridDim.x * blockDim.x) {
+        if (i < t.nMask) {
+            const float u = sqrtf((float)(t.qIn + i));
+            t.mask[i] = i ? 1.f - (0.5f - 0.5f * cospif((u - t.r) / t.ew)) : 1.f;
+        }
+        if (t.A && i < t.K) {
+            const int k = t.iCol[i], b = k / t.cols, c0 = b * t.cols;
+            const int nc = min(t.cols, t.maxCol + 1 - c0);
+            const int r = t.iRow[i], y = r < 0 ? r + N : r;
+            t.slot[i] = (b << 20) + (y < N / 2 ? y * t.W : (y - N / 2) * t.W + nc) + k - c0;
+        }
+    }
     const float* im = img + l * N * N;
     const int half = N / 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const float pivot = im[0];
-    double s1 = 0.0, s2 = 0.0, cnt = 0.0;
-    for (int y = warp; y < N; y += nw) {
-        const int j = y - half;
-        const float* row = im + (size_t)y * N;
-        float a1 = 0.f, a2 = 0.f;
-        int c = 0;
-        for (int x = lane; x < N; x += 32) {
-            const int i = x - half;
-            if ((long long)(i * i + j * j) > bgAbove) {
-                const float d = row[x] - pivot;
+    for (int y = threadIdx.x; y < (N + 3) / 4 * 4; y += blockDim.x) {
+        const int j = y - half, q = bgAbove - j * j;
+        int h = -1;                              // the row inside: |i| <= h
+        if (q >= 0) {
+            h = (int)sqrtf((float)q);
+            while (h * h > q) h--;
+            while ((h + 1) * (h + 1) <= q) h++;
+        }
+        rows[y] = y >= N   ? make_int2(0, 0)
+                  : h < 0 ? make_int2(N, 0)
+                          : make_int2(max(half - h, 0), max(half - h - 1, 0));
+    }
+    __syncthreads();
+    Total t1{0.f, 0.f}, t2{0.f, 0.f};
+    for (int y0 = 4 * warp; y0 < N; y0 += 4 * nw) {
+        int left[4], n[4], most = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int2 r = rows[y0 + k];
+            left[k] = r.x;
+            n[k] = r.x + r.y;
+            most = max(most, n[k]);
+        }
+        for (int e = lane; e < most; e += 64) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int f = e + 32 * (k & 1), r = k >> 1;
+                const int x = (y0 + r) * N + (f < left[r] ? f : N - n[r] + f);
+                v[k] = __ldg(im + (f < n[r] ? x : 0));
+            }
+            float a1 = 0.f, a2 = 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float d = v[k] - pivot;
                 a1 += d;
                 a2 = fmaf(d, d, a2);
-                c++;
             }
+            t1.add(a1);
+            t2.add(a2);
         }
-        s1 += a1;
-        s2 += a2;
-        cnt += c;
     }
-    s1 = prep_block_sum(s1, red);
-    s2 = prep_block_sum(s2, red);
-    cnt = prep_block_sum(cnt, red);
+    t1.warp_sum();
+    t2.warp_sum();
+    if (lane == 0) {
+        part[0][warp] = t1;
+        part[1][warp] = t2;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
+        double s1 = 0.0, s2 = 0.0;
+        for (int w = 0; w < nw; w++) {
+            s1 += part[0][w].value();
+            s2 += part[1][w].value();
+        }
         const double mu = s1 / cnt;                 // mean about the pivot
         const double ss = fmax(s2 - s1 * mu, 0.0);  // sum of (x - m)^2
         const double sd = sqrt(ss / (cnt - 1.0));
-        st[3 * l] = pivot + mu;
-        st[3 * l + 1] = sd;
         // sum of ((x - m) / sd)^2 over the background, over (n - 1)
-        st[3 * l + 2] = sqrt(ss / (sd * sd) / (cnt - 1.0));
+        const double o[4] = {pivot + mu, sd, sqrt(ss / (sd * sd) / (cnt - 1.0)), 1.0 / sd};
+        for (int i = 0; i < 4; i++) {
+            st[4 * l + i] = o[i];
+            if (st32 && i < 3) st32[3 * l + i] = (float)o[i];
+        }
     }
 }
 
-__global__ void k_stats_f32(const double* __restrict__ st, int n, float* __restrict__ out)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n; i += gridDim.x * blockDim.x)
-        out[i] = (float)st[i];
-}
-
-// stdN: the given value, or the mean of the images' sN; out = (stdN, 1 / stdN).
-__global__ void k_stdn(const double* __restrict__ st, int n, float given, double* __restrict__ out)
+// stdN: the given value, or the mean of the images' sN; then every image's
+// scaling by 1 / (s stdN).  One CTA.
+__global__ void __launch_bounds__(256)
+k_stdn(const double* __restrict__ st, int n, float given, Scaling* __restrict__ out)
 {
     __shared__ double red[32];
     double s = 0.0;
-    for (int l = threadIdx.x; l < n; l += blockDim.x) s += st[3 * (size_t)l + 2];
+    for (int l = threadIdx.x; l < n; l += blockDim.x) s += st[4 * (size_t)l + 2];
     s = prep_block_sum(s, red);
-    if (threadIdx.x == 0) {
-        out[0] = given > 0.f ? (double)given : s / n;
-        out[1] = 1.0 / out[0];
+    const double scale = 1.0 / (given > 0.f ? (double)given : s / n);
+    for (int l = threadIdx.x; l < n; l += blockDim.x) {
+        const double mean = st[4 * (size_t)l], f = scale * st[4 * (size_t)l + 3];
+        const float m = (float)mean;
+        out[l] = {m, (float)f, (float)((m - mean) * f)};
     }
 }
 
 constexpr int kPrepRows = 4;   // image rows per CTA of k_prep_image
 
-// Normalise, mask and scale one image row, written with the image's centre
-// at index 0.
-__global__ void k_prep_image(const float* __restrict__ img, int N, float r, float ew, int mask,
-                             const double* __restrict__ st, const double* __restrict__ stdN,
-                             float* __restrict__ out)
+// Normalise, mask and scale rows of an image, written with the image's centre
+// at index 0, for the library's transform.  CTA (kPrepRows rows, image l);
+// threads over the columns, a thread's rows loaded together; pixels outside
+// the mask are not read.
+__global__ void k_prep_image(const float* __restrict__ img, int N, const SoftMask mask,
+                             const Scaling* __restrict__ scaling, float* __restrict__ out)
 {
     const size_t l = blockIdx.y;
-    const float m = (float)st[3 * l], sd = (float)st[3 * l + 1];
-    const float scale = (float)stdN[1];
-    const int half = N / 2;
-    // CTA (kPrepRows rows, image l); threads over the rows' columns
-    const int y1 = min(N, (int)(blockIdx.x + 1) * kPrepRows);
-    for (int y = blockIdx.x * kPrepRows; y < y1; y++)
+    const Scaling sc = scaling[l];
+    const int half = N / 2, y0 = blockIdx.x * kPrepRows;
+    const float* im = img + l * N * N;
     for (int x = threadIdx.x; x < N; x += blockDim.x) {
-        const int q = y * N + x;
-        const int i = x - half, j = y - half;
-        float v = (img[l * N * N + q] - m) / sd;
-        if (mask) {
-            const float u = sqrtf((float)(i * i + j * j));
-            if (u > r + ew)
-                v = 0.f;
-            else if (u >= r) {
-                const float w = 0.5f - 0.5f * cospif((u - r) / ew);
-                v = v * (1.f - w);
-            }
+        const int i = x - half;
+        float v[kPrepRows];
+        int q[kPrepRows];
+#pragma unroll
+        for (int k = 0; k < kPrepRows; k++) {
+            const int j = min(y0 + k, N - 1) - half;
+            q[k] = i * i + j * j;
+            v[k] = __ldg(im + (q[k] <= mask.qOut ? (size_t)(j + half) * N + x : 0));
         }
-        const int ci = i < 0 ? i + N : i, cj = j < 0 ? j + N : j;
-        out[l * N * N + (size_t)cj * N + ci] = v * scale;
+#pragma unroll
+        for (int k = 0; k < kPrepRows; k++) {
+            const int j = y0 + k - half;
+            const int ci = i < 0 ? i + N : i, cj = j < 0 ? j + N : j;
+            if (y0 + k < N)
+                out[l * N * N + (size_t)cj * N + ci] = masked(scaled(sc, v[k]), q[k], mask, mask.tab);
+        }
     }
+}
+
+// Normalisation, mask, 2-D transform and pixel gather of one image by one CTA,
+// the transform on chip (tg3_fft.cuh has its two-step form; N = A B, A even).
+// A warp holds one line, or two of up to 16 lanes, and needs no other warp:
+//   rows: the rows y and y + N/2 of the centred image are the real and the
+//     imaginary part of one line; of its transform Z the columns k and N - k of
+//     this CTA's range c0 <= k < c0 + cols stay in shared memory;
+//   columns: a lane's inputs of column k at y and y + N/2 are (Z[k] +
+//     conj Z[N - k]) / 2 and (Z[k] - conj Z[N - k]) / 2i of that line, so the
+//     two rows part on the way in; the result takes the column's place;
+//   then the pixels are read out in the list's order.
+// Images whose columns do not fit take several CTAs, each with a range of the
+// columns and all rows; they meet in L2.  Bound by instruction issue at one CTA an
+// SM (115,000 warp instructions an image of 256^2 at 0.46 a cycle and
+// scheduler); the image is read once, inside the mask, and only the list's
+// pixels are written.  1,024 images of 256^2, 9,930 pixels: 200 us, where the
+// normalised images, the library's two transform kernels and the gather took
+// 495.
+struct PrepFt {
+    const float* img;
+    int A, B, lanes;         // lanes of a line: 16 or 32
+    int ex;                  // exchange buffer of a line
+    int cols, maxCol, W;     // columns of a CTA, the last one of the list, row pitch
+    SoftMask mask;
+    const float2* tw;
+    const Scaling* scaling;
+    const int* slot;         // (CTA of the image << 20) + place of a pixel
+    int K;
+    float2* dat;
+};
+
+#define TG3_RADIX_A(X) X(6) X(8) X(10) X(12) X(14) X(16) X(18) X(20)
+#define TG3_RADIX_B(X) \
+    X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(18) X(20)
+
+template <int R>
+struct Radix {
+    static constexpr int value = R;
+};
+
+template <class F>
+__device__ __forceinline__ void with_a(int r, F f)
+{
+    switch (r) {
+#define X(n) case n: f(Radix<n>()); break;
+        TG3_RADIX_A(X)
+#undef X
+    }
+}
+template <class F>
+__device__ __forceinline__ void with_b(int r, F f)
+{
+    switch (r) {
+#define X(n) case n: f(Radix<n>()); break;
+        TG3_RADIX_B(X)
+#undef X
+    }
+}
+
+using fft::c64;
+
+// first step's output of item t to the line's exchange buffer
+template <int R>
+__device__ __forceinline__ void prep_exchange(c64 (&v)[R], c64* xb, const float2* tw, int B, int t)
+{
+    fft::dft<R>(v);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const float2 w = tw[r * B + t];
+        xb[r * (B | 1) + t] = r ? fft::times(v[r], w.x, w.y) : v[r];
+    }
+}
+
+// x, as a value of this iteration: what hangs on it is worked out again instead
+// of being kept in registers over the loop, where it does not fit
+__device__ __forceinline__ int again(int x)
+{
+    asm volatile("" : "+r"(x));
+    return x;
+}
+
+// the two rows' pixels of item t of line y
+struct PrepRows {
+    float a[20], b[20];
+};
+
+template <int R>
+__device__ __forceinline__ void prep_load(const PrepFt& p, size_t l, int N, int y, int t, PrepRows& v)
+{
+    const int half = N / 2, B = p.B;
+    // rows of the coordinates y and y - N/2, from column 0
+    const float* r0 = p.img + (l * N + y + half) * N + half;
+    const float* r1 = p.img + (l * N + y) * N + half;
+    const int q0 = y * y, q1 = (half - y) * (half - y);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = t + (r < R / 2 ? r : r - R) * B;
+        v.a[r] = __ldg(r0 + (i * i + q0 <= p.mask.qOut ? i : 0));
+        v.b[r] = __ldg(r1 + (i * i + q1 <= p.mask.qOut ? i : 0));
+    }
+}
+
+__global__ void __launch_bounds__(512, 1) k_prep_ft(const PrepFt p)
+{
+    extern __shared__ __align__(16) c64 psm[];
+    const int A = p.A, B = p.B, N = A * B, half = N / 2, W = p.W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int per = 32 / p.lanes, sub = lane / p.lanes;
+    c64* big = psm;
+    c64* xb = big + half * W + (warp * per + sub) * p.ex;
+    float2* tw = reinterpret_cast<float2*>(big + half * W + nw * per * p.ex);
+    float* tab = reinterpret_cast<float*>(tw + N);
+    const size_t l = blockIdx.y;
+    // the first rows' pixels are on their way while the tables are copied, the
+    // next ones' behind each line's second step
+    PrepRows px;
+    with_a(A, [&](auto radix) {
+        constexpr int R = decltype(radix)::value;
+        const int t = lane % p.lanes;
+        if (t < B) prep_load<R>(p, l, N, min(warp * per + sub, half - 1), t, px);
+    });
+    for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = p.tw[i];
+    for (int i = threadIdx.x; i <= p.mask.qOut - p.mask.qIn; i += blockDim.x) tab[i] = p.mask.tab[i];
+    const int c0 = blockIdx.x * p.cols, nc = min(p.cols, p.maxCol + 1 - c0);
+    Scaling sc = p.scaling[l];
+    sc.f *= 0.5f;                                // for the columns' halves
+    sc.c *= 0.5f;
+    __syncthreads();
+
+    for (int base = warp * per; base < half; base += nw * per) {
+        const int y = base + sub, t = again(lane % p.lanes);
+        const int yl = min(y, half - 1), next = min(y + nw * per, half - 1);
+        const int q0 = yl * yl, q1 = (half - yl) * (half - yl);
+        with_a(A, [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            if (t >= B) return;
+            c64 v[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int i = t + (r < R / 2 ? r : r - R) * B;
+                v[r] = fft::pack(masked(scaled(sc, px.a[r]), i * i + q0, p.mask, tab),
+                                 masked(scaled(sc, px.b[r]), i * i + q1, p.mask, tab));
+            }
+            prep_exchange<R>(v, xb, tw, B, t);
+            prep_load<R>(p, l, N, next, t, px);
+        });
+        __syncwarp();
+        with_b(B, [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            if (t >= A || y >= half) return;
+            c64 o[R];
+#pragma unroll
+            for (int s = 0; s < R; s++) o[s] = xb[t * (R | 1) + s];
+            fft::dft<R>(o);
+            c64* row = big + y * W;
+#pragma unroll
+            for (int s = 0; s < R; s++) {
+                const int k = t + A * s, d = k - c0, e = (k ? N - k : 0) - c0;
+                if (d >= 0 && d < nc) row[d] = o[s];
+                if (e >= 0 && e < nc) row[nc + e] = o[s];
+            }
+        });
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int base = warp * per; base < nc; base += nw * per) {
+        const int k = base + sub, kl = min(k, nc - 1), t = again(lane % p.lanes);
+        with_a(A, [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            if (t >= B) return;
+            c64 v[R];
+#pragma unroll
+            for (int r = 0; r < R / 2; r++) {
+                const c64* row = big + (t + r * B) * W + kl;
+                const float2 a = fft::unpack(row[0]), b = fft::unpack(row[nc]);
+                v[r] = fft::pack(a.x + b.x, a.y - b.y);            // the 1/2 is in the scaling
+                v[r + R / 2] = fft::pack(a.y + b.y, b.x - a.x);
+            }
+            prep_exchange<R>(v, xb, tw, B, t);
+        });
+        __syncwarp();
+        with_b(B, [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            if (t >= A || k >= nc) return;
+            c64 o[R];
+#pragma unroll
+            for (int s = 0; s < R; s++) o[s] = xb[t * (R | 1) + s];
+            fft::dft<R>(o);
+#pragma unroll
+            for (int s = 0; s < R; s++) {
+                const int y = t + A * s;
+                big[y < half ? y * W + k : (y - half) * W + nc + k] = o[s];
+            }
+        });
+        __syncwarp();
+    }
+    __syncthreads();
+    float2* dat = p.dat + l * p.K;
+    constexpr int G = 8;
+    for (int i0 = threadIdx.x; i0 < p.K; i0 += G * blockDim.x) {
+        int at[G];
+#pragma unroll
+        for (int g = 0; g < G; g++) at[g] = __ldg(p.slot + min(i0 + g * (int)blockDim.x, p.K - 1));
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const int i = i0 + g * blockDim.x;
+            if (i < p.K && at[g] >> 20 == (int)blockIdx.x)
+                dat[i] = fft::unpack(big[at[g] & 0xfffff]);
+        }
+    }
+}
+
+// The factors of N (A even, both in the kernel's lists, the nearest to each
+// other), and the launch that takes the fewest CTAs an image (each repeats the
+// rows: 1,000 images of 256^2 take 200 us with one and, for 102 columns, 314
+// with two, the separate kernels 500), then the most warps an SM.  0 where N has
+// no such factors (254: the library's transform by 127 stays) or four CTAs
+// cannot hold the columns.
+struct PrepLaunch {
+    int A = 0, B = 0, lanes = 0, ex = 0, cols = 0, W = 0, blocks = 0, threads = 0;
+    size_t smem = 0;
+};
+
+PrepLaunch prep_launch(int N, int maxCol, int nMask)
+{
+    PrepLaunch o;
+    const int as[] = {
+#define X(n) n,
+        TG3_RADIX_A(X)};
+    const int bs[] = {TG3_RADIX_B(X)};
+#undef X
+    for (int a : as)
+        for (int b : bs)
+            if (a * b == N && (!o.A || std::abs(a - b) < std::abs(o.A - o.B))) o.A = a, o.B = b;
+    if (!o.A) return o;
+    o.lanes = std::max(o.A, o.B) <= 16 ? 16 : 32;
+    o.ex = o.A * (o.B | 1);
+    for (o.blocks = 1; o.blocks <= 4; o.blocks++) {
+        o.cols = (maxCol + o.blocks) / o.blocks;
+        o.W = 2 * o.cols | 1;                      // odd: a column's rows spread over the banks
+        auto bytes = [&](int warps) {
+            return sizeof(c64) * ((size_t)N / 2 * o.W + (size_t)warps * (32 / o.lanes) * o.ex + N) +
+                   sizeof(float) * nMask;
+        };
+        int warps = 2 * (bytes(8) + 1024) <= kSmemSm ? 8 : 16;
+        while (warps >= 8 && bytes(warps) > kSmemCta) warps -= 4;
+        if (warps >= 8) {
+            o.threads = 32 * warps;
+            o.smem = bytes(warps);
+            return o;
+        }
+    }
+    return PrepLaunch();
 }
 
 // dat[l][p] = FT[l][iRow mod N][iCol]
@@ -478,40 +850,75 @@ extern "C" int tg3_prepare_images_d(tg3_ctx* c, const float* img, int nImg, int 
     if (maskRadiusPx >= N / 2 * 1.4142135f)
         return fail(TG3_ERR_ARG, "mask radius leaves no background pixels");
     const int K = c->px.K;
-    const int IB = std::min(nImg, 2048);
-    const size_t img2 = (size_t)N * N, ft2 = (size_t)N * (N / 2 + 1);
+    const float r = maskRadiusPx, ew = 6.0f;
+    // the background's pixels, and the mask's edge in squared radii, compared as
+    // the FP32 radii u = sqrt(q) are: u < r inside, u > r + ew outside
+    const int half = N / 2, bgAbove = (int)std::floor((double)r * (double)r);
+    long long cnt = 0;
+    for (int j = -half; j < half; j++) {
+        const long long q = (long long)bgAbove - (long long)j * j;
+        int h = q < 0 ? -1 : (int)std::sqrt((double)q);
+        while (h >= 0 && (long long)h * h > q) h--;
+        while (q >= 0 && (h + 1LL) * (h + 1) <= q) h++;
+        cnt += h < 0 ? N : std::max(half - h, 0) + std::max(half - h - 1, 0);
+    }
+    SoftMask sm{nullptr, 2 * half * half, 2 * half * half};
+    if (mask) {
+        sm.qIn = (int)std::min((double)r * r + 2, 2.0 * half * half);
+        while (sm.qIn > 0 && !(std::sqrt((float)sm.qIn) < r)) sm.qIn--;
+        sm.qOut = (int)std::min(((double)r + ew) * ((double)r + ew) + 2, 2.0 * half * half);
+        while (sm.qOut > sm.qIn && std::sqrt((float)sm.qOut) > r + ew) sm.qOut--;
+    }
+    const int nMask = sm.qOut - sm.qIn + 1;
+    const PrepLaunch pl = prep_launch(N, std::min(c->px.maxAbs, half), nMask);
+    const int IB = std::min(nImg, pl.A ? 65535 : 2048);
+    const size_t img2 = (size_t)N * N, ft2 = (size_t)N * (half + 1);
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t oSt = 0, oN = up(sizeof(double) * 3 * (size_t)nImg), oR = oN + 256,   // oN: 2 doubles
-                 oF = up(oR + sizeof(float) * img2 * IB), total = oF + sizeof(float2) * ft2 * IB;
+    const size_t oSt = 0, oN = up(sizeof(double) * 4 * (size_t)nImg),
+                 oM = oN + up(sizeof(Scaling) * (size_t)nImg), oT = oM + up(sizeof(float) * nMask),
+                 oL = oT + up(sizeof(float2) * (pl.A ? N : 0)),
+                 oR = oL + up(sizeof(int) * (pl.A ? K : 0)),
+                 oF = up(oR + (pl.A ? 0 : sizeof(float) * img2 * IB)),
+                 total = oF + (pl.A ? 0 : sizeof(float2) * ft2 * IB);
     char* b = (char*)ws_get(c, WS_PREP, total, &st);
     if (!b) return st;
     double* stv = (double*)(b + oSt);
-    double* sN = (double*)(b + oN);
+    Scaling* sc = (Scaling*)(b + oN);
     float* real = (float*)(b + oR);
     cufftComplex* ft = (cufftComplex*)(b + oF);
     cudaStream_t s = c->stream;
-    const float r = maskRadiusPx;
-    k_bg_stats<<<nImg, 256, 0, s>>>(img, N, (long long)std::floor((double)r * (double)r), stv);
+    sm.tab = (float*)(b + oM);
+    const int maxCol = std::min(c->px.maxAbs, half);
+    const PrepTables tabs{(float*)(b + oM), sm.qIn, nMask, r, ew, (float2*)(b + oT), pl.A, pl.B,
+                          (int*)(b + oL), c->px.iCol, c->px.iRow, pl.A ? K : 0, pl.cols, maxCol,
+                          pl.W};
+    k_bg_stats<<<nImg, 256, sizeof(int2) * up(N), s>>>(img, N, bgAbove, (double)cnt, stv, stats, tabs);
     TG3_LAUNCH_CHECK("background statistics");
-    k_stdn<<<1, 256, 0, s>>>(stv, nImg, stdN, sN);
+    k_stdn<<<1, 256, 0, s>>>(stv, nImg, stdN, sc);
     TG3_LAUNCH_CHECK("noise level");
+    if (pl.A)
+        TG3_CUDA(cudaFuncSetAttribute(k_prep_ft, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSmemCta));
     for (int l0 = 0; l0 < nImg; l0 += IB) {
         const int n = std::min(IB, nImg - l0);
+        float2* out = reinterpret_cast<float2*>(dat) + (size_t)l0 * K;
+        if (pl.A) {
+            const PrepFt f{img + (size_t)l0 * img2, pl.A, pl.B, pl.lanes, pl.ex, pl.cols,
+                           maxCol, pl.W, sm, tabs.tw, sc + l0, tabs.slot, K, out};
+            k_prep_ft<<<dim3(pl.blocks, n), pl.threads, pl.smem, s>>>(f);
+            TG3_LAUNCH_CHECK("normalise, mask, transform and gather");
+            continue;
+        }
         k_prep_image<<<dim3((N + kPrepRows - 1) / kPrepRows, n), std::min(N, 256), 0, s>>>(
-            img + (size_t)l0 * img2, N, r, 6.0f, mask, stv + 3 * (size_t)l0, sN, real);
+            img + (size_t)l0 * img2, N, sm, sc + l0, real);
         TG3_LAUNCH_CHECK("normalise and mask");
         cufftHandle h;
         if ((st = get_plan(c, N, n, &h))) return st;
         if (cufftSetStream(h, s) != CUFFT_SUCCESS || cufftExecR2C(h, real, ft) != CUFFT_SUCCESS)
             return fail(TG3_ERR_CUDA, "cuFFT forward transform failed");
         k_gather_pixels<<<dim3((K + 255) / 256, n), 256, 0, s>>>(
-            reinterpret_cast<const float2*>(ft), N, c->px.iCol, c->px.iRow, K,
-            reinterpret_cast<float2*>(dat) + (size_t)l0 * K);
+            reinterpret_cast<const float2*>(ft), N, c->px.iCol, c->px.iRow, K, out);
         TG3_LAUNCH_CHECK("pixel gather");
-    }
-    if (stats) {
-        k_stats_f32<<<(3 * nImg + 255) / 256, 256, 0, s>>>(stv, nImg, stats);
-        TG3_LAUNCH_CHECK("statistics");
     }
     return TG3_OK;
 }
