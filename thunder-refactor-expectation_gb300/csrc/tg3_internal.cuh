@@ -60,19 +60,17 @@ __host__ __device__ __forceinline__ int cubes_x(int vdim) { return (vdim / 2 + 1
 __host__ __device__ __forceinline__ int cubes_yz(int vdim) { return (vdim + 31) / 32; }
 
 // Per-axis terms of a block's index: block(x, y, z) = tx[x] + ty[y + vdim/2]
-// + tz[z + vdim/2] for x in [0, vdim/2], y, z in [-vdim/2, vdim/2), the y and
-// z tables absorbing the wrap of negative rows.  tx has vdim/2 + 1 entries,
+// + tz[z + vdim/2] for x in [0, vdim/2], y, z in [-vdim/2, vdim/2).  tx has vdim/2 + 1 entries,
 // ty and tz vdim each; filled by the threads of a CTA (x-stride blockDim.x).
 __device__ __forceinline__ void fill_brick_tables(int vdim, int* tx, int* ty, int* tz)
 {
-    const int nx = vdim / 2 + 1, half = vdim / 2;
+    const int nx = vdim / 2 + 1;
     const int nxc = cubes_x(vdim), nyc = cubes_yz(vdim);
     for (int j = threadIdx.x; j < nx; j += blockDim.x)
         tx[j] = (j >> 5) * 32768 + ((j >> 3) & 3) * 512 + (j & 7);
     for (int j = threadIdx.x; j < vdim; j += blockDim.x) {
-        const int w = j - half < 0 ? j + half : j - half;
-        ty[j] = (w >> 5) * nxc * 32768 + ((w >> 3) & 3) * 2048 + (w & 7) * 8;
-        tz[j] = (w >> 5) * nyc * nxc * 32768 + ((w >> 3) & 3) * 8192 + (w & 7) * 64;
+        ty[j] = (j >> 5) * nxc * 32768 + ((j >> 3) & 3) * 2048 + (j & 7) * 8;
+        tz[j] = (j >> 5) * nyc * nxc * 32768 + ((j >> 3) & 3) * 8192 + (j & 7) * 64;
     }
 }
 

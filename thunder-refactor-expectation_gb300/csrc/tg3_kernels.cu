@@ -169,7 +169,9 @@ __global__ void k_ctf(const float* __restrict__ attr, int nImg, float px, int id
     }
 }
 
-// Placement of voxel (z, y, x)'s corner block: the volume is cut into
+// Placement of the corner block of voxel (z, y, x), z and y counted from the
+// lowest coordinate -vdim / 2 (so that a sample's index needs no wrap): the
+// volume is cut into
 // cubes of 32^3 voxels (32768 blocks = 2 MB, one large page each, cubes in
 // z, y, x order), each cube into 4^3 bricks of 8^3 voxels, voxels x-fastest
 // within a brick.  A projection's samples within one pixel band then touch a
@@ -201,7 +203,9 @@ __global__ void k_volume_blocks(const float2* __restrict__ vol, int vdim,
         const int x = (int)(i % nx);
         const int y = (int)((i / nx) % vdim);
         const int z = (int)(i / ((size_t)nx * vdim));
-        const size_t d = brick_index(x, y, z, nxc, nyc);
+        const int half = vdim / 2;
+        const size_t d = brick_index(x, y < half ? y + half : y - half,
+                                     z < half ? z + half : z - half, nxc, nyc);
         const int y1 = y + 1 == vdim ? 0 : y + 1;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
@@ -472,9 +476,7 @@ k_project_lane(float4* const* __restrict__ volTable, const int* __restrict__ cls
             fw[u][2] = z - zf;
             unsigned blk;
             if (kArith) {
-                // brick_index with the rows' and slabs' wrap of negative indices
-                const int yy = y0 < 0 ? y0 + vdim : y0;
-                const int zz = z0 < 0 ? z0 + vdim : z0;
+                const int yy = y0 + half, zz = z0 + half;
                 blk = (unsigned)((((zz >> 5) * nyc + (yy >> 5)) * nxc + (x0 >> 5)) * 32768
                                  + ((((zz >> 3) & 3) * 4 + ((yy >> 3) & 3)) * 4 + ((x0 >> 3) & 3)) * 512
                                  + ((zz & 7) * 8 + (yy & 7)) * 8 + (x0 & 7));
@@ -549,6 +551,41 @@ k_project_lane(float4* const* __restrict__ volTable, const int* __restrict__ cls
 // the pair form's sum).  (Recomputing the partner's fractions from its
 // coordinates instead of receiving them by three shuffles measured slower:
 // 8.99 against 8.56 ms per 128 particles at box 256.)
+// Block index and fractions of a sample, without tables and conversions: the
+// floor comes out of an addition rounded down (x + 1.5 2^23 has the integer part
+// of x in its low bits), the index fields (brick_index) out of shifted copies
+// of those bits, x = a + 8 b + 32 c -> a + 512 b + 32768 c and so on, with all
+// offsets in one constant.  A coordinate outside the volume (not a number) is
+// held to the blocks there are.
+struct BrickIndex {
+    unsigned yc, zc, offset, last;
+    float yMagic;
+    __device__ __forceinline__ explicit BrickIndex(int vdim)
+    {
+        const unsigned nxc = cubes_x(vdim), nyc = cubes_yz(vdim), bias = 0x4b400000u;
+        yc = nxc * 32768u - 8192u;
+        zc = nxc * nyc * 32768u - 32768u;
+        yMagic = 12582912.f + (float)(vdim / 2);
+        last = nxc * nyc * nyc * 32768u - 1u;
+        offset = 0u - (bias + 504u * (bias >> 3) + 30720u * (bias >> 5)) -
+                 (8u * bias + 1984u * (bias >> 3) + yc * (bias >> 5)) -
+                 (64u * bias + 7680u * (bias >> 3) + zc * (bias >> 5));
+    }
+    __device__ __forceinline__ unsigned operator()(float x, float y, float z, float (&f)[3]) const
+    {
+        const float tx = __fadd_rd(x, 12582912.f), ty = __fadd_rd(y, yMagic),
+                    tz = __fadd_rd(z, yMagic);
+        f[0] = x - (tx - 12582912.f);
+        f[1] = y - (ty - yMagic);
+        f[2] = z - (tz - yMagic);
+        const unsigned bx = __float_as_uint(tx), by = __float_as_uint(ty), bz = __float_as_uint(tz);
+        const unsigned b = offset + bx + 504u * (bx >> 3) + 30720u * (bx >> 5) + 8u * by +
+                           1984u * (by >> 3) + yc * (by >> 5) + 64u * bz + 7680u * (bz >> 3) +
+                           zc * (bz >> 5);
+        return min(b, last);
+    }
+};
+
 template <bool kArith, int G>
 __global__ void __launch_bounds__(256, 4)
 k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls,
@@ -558,8 +595,11 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
                const float* __restrict__ sigRcp, const float* __restrict__ ctf,
                float* __restrict__ nrmPart, int* __restrict__ flag, long long splitLo)
 {
-    __shared__ float m[G][9];
+    __shared__ __align__(16) float m[G][8];      // rows 0 - 2, columns 0 and 1
     __shared__ float red[G][8];
+    // a warp's norm terms of every rotation, LPR lanes of it a rotation at the end
+    constexpr int LPR = 32 / G, kPitch = 32 + LPR;
+    __shared__ float part[8][G * kPitch];
     const int g = blockIdx.x % nGroups;
     const int chunk = (blockIdx.x / nGroups) % nChunks;
     const int l = blockIdx.x / (nGroups * nChunks);
@@ -568,12 +608,15 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
     const size_t row0 = (size_t)l * rowsPerParticle + r0;
     extern __shared__ int tab[];
     const int half = vdim / 2;
-    const int nxc = cubes_x(vdim), nyc = cubes_yz(vdim);
     int* tx = tab;
     int* ty = tab + vdim / 2 + 1;
     int* tz = ty + vdim;
     if (!kArith) fill_brick_tables(vdim, tx, ty, tz);
-    if (threadIdx.x < 9 * nRot) m[threadIdx.x / 9][threadIdx.x % 9] = mf[9 * row0 + threadIdx.x];
+    if (threadIdx.x < 6 * nRot) {
+        const int i = threadIdx.x / 6, e = threadIdx.x % 6;
+        m[i][e] = mf[9 * (row0 + i) + e / 2 * 3 + e % 2];
+    }
+    const BrickIndex bi(vdim);
     __syncthreads();
     const int nOut = ldo / 2;
     const int h = threadIdx.x & 1;
@@ -623,31 +666,27 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll 1
     for (int i = 0; i < nRot; i++) {   // nRot is uniform across the CTA
-        const float* mm = m[i];
+        const float4 m01 = *reinterpret_cast<const float4*>(m[i]);
+        const float2 m2 = *reinterpret_cast<const float2*>(m[i] + 4);
         float acc = 0.f;
         float fo[kLaneU][3], fp[kLaneU][3];   // own and partner fractions
         bool cj[kLaneU];
         unsigned bo[kLaneU], bp[kLaneU];      // own and partner block index
 #pragma unroll
         for (int u = 0; u < kLaneU; u++) {
-            float x = mm[0] * pa[u] + mm[1] * pb[u];
-            float y = mm[3] * pa[u] + mm[4] * pb[u];
-            float z = mm[6] * pa[u] + mm[7] * pb[u];
+            float x = m01.x * pa[u] + m01.y * pb[u];
+            float y = m01.z * pa[u] + m01.w * pb[u];
+            float z = m2.x * pa[u] + m2.y * pb[u];
             cj[u] = x < 0.f;
             if (cj[u]) { x = -x; y = -y; z = -z; }
-            const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
-            const int x0 = (int)xf, y0 = (int)yf, z0 = (int)zf;
-            fo[u][0] = x - xf;
-            fo[u][1] = y - yf;
-            fo[u][2] = z - zf;
             if (kArith) {
-                const int yy = y0 < 0 ? y0 + vdim : y0;
-                const int zz = z0 < 0 ? z0 + vdim : z0;
-                bo[u] = (unsigned)((((zz >> 5) * nyc + (yy >> 5)) * nxc + (x0 >> 5)) * 32768
-                                   + ((((zz >> 3) & 3) * 4 + ((yy >> 3) & 3)) * 4 + ((x0 >> 3) & 3)) * 512
-                                   + ((zz & 7) * 8 + (yy & 7)) * 8 + (x0 & 7));
+                bo[u] = bi(x, y, z, fo[u]);
             } else {
-                bo[u] = (unsigned)(tx[x0] + ty[y0 + half] + tz[z0 + half]);
+                const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
+                fo[u][0] = x - xf;
+                fo[u][1] = y - yf;
+                fo[u][2] = z - zf;
+                bo[u] = (unsigned)(tx[(int)xf] + ty[(int)yf + half] + tz[(int)zf + half]);
             }
             bp[u] = __shfl_xor_sync(0xffffffffu, bo[u], 1);
 #pragma unroll
@@ -703,12 +742,23 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
                 }
             }
         }
-        if (nrmPart) {
-            acc = warp_sum(acc);
-            if (lane == 0) red[i][wid] = acc;
-        }
+        part[wid][i * kPitch + lane] = acc;
     }
     if (nrmPart) {
+        // the sums over the lanes of all rotations together, in warp_sum's order
+        // (lanes 16 apart, then 8, ...): LPR lanes a rotation
+        __syncwarp();
+        const int j = lane / LPR;
+        float v[G];
+#pragma unroll
+        for (int k = 0; k < G; k++) v[k] = part[wid][j * kPitch + lane % LPR + LPR * k];
+#pragma unroll
+        for (int w = G / 2; w; w >>= 1)
+#pragma unroll
+            for (int k = 0; k < w; k++) v[k] += v[k + w];
+#pragma unroll
+        for (int o = LPR / 2; o; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        if (lane % LPR == 0) red[j][wid] = v[0];
         __syncthreads();
         if (threadIdx.x < nRot) {
             float s = 0.f;
@@ -2463,7 +2513,7 @@ cudaError_t launch_project(float4* const* volTable, const int* cls, const float4
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tabBytes);
         if (e != cudaSuccess) return e;
     }
-    kern<<<(unsigned)grid, 256, tabBytes, st>>>(volTable, cls, vol, vdim, pf, mf, rowsPerParticle,
+    kern<<<(unsigned)grid, 256, form == 4 ? 0 : tabBytes, st>>>(volTable, cls, vol, vdim, pf, mf, rowsPerParticle,
                                                 nGroups, nChunks, iCol, iRow, K, out, ldo, sigRcp,
                                                 ctf, nrm ? nrmPart : nullptr, flag, splitLo);
     e = cudaGetLastError();
