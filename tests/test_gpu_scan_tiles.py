@@ -33,7 +33,7 @@ def ctx():
 
 @pytest.mark.parametrize("nImg,nR,nT", [(1, 1, 1), (3, 127, 9), (5, 129, 31), (7, 300, 32),
                                         (2, 256, 33), (9, 640, 49), (310, 128, 25), (1, 1300, 256),
-                                        (40, 77, 3), (306, 515, 64)])
+                                        (40, 77, 3), (306, 515, 64), (3, 70, 300)])
 def test_best_and_marginals(ctx, nImg, nR, nT):
     iCol, _, _, _ = synth.pixel_index(32, 9, 1)
     K = len(iCol)

@@ -540,17 +540,6 @@ k_project_lane(float4* const* __restrict__ volTable, const int* __restrict__ cls
     }
 }
 
-// Lane pairs that share loads but not the coordinate work (forms 3 and 4).
-// Every lane finds the block index and fractions of its own pixel (as in the
-// one-lane form: once per sample), then a pair swaps them by one shuffle
-// each.  The pair's two loads read pixel A's block (lane 0 slab z0, lane 1
-// slab z0 + 1) and then pixel B's, so every load instruction takes whole
-// 64-byte blocks, one L1 wavefront per pixel as in the lane-pair form.
-// Each lane forms its slab's share of both pixels; lane 0 keeps A and lane 1
-// B, the other share arriving by shuffle (slab z0's share plus slab z0 + 1's,
-// the pair form's sum).  (Recomputing the partner's fractions from its
-// coordinates instead of receiving them by three shuffles measured slower:
-// 8.99 against 8.56 ms per 128 particles at box 256.)
 // Block index and fractions of a sample, without tables and conversions: the
 // floor comes out of an addition rounded down (x + 1.5 2^23 has the integer part
 // of x in its low bits), the index fields (brick_index) out of shifted copies
@@ -586,6 +575,23 @@ struct BrickIndex {
     }
 };
 
+// Lane pairs that share loads but not the coordinate work (forms 3 and 4).
+// Every lane finds the block index and fractions of its own pixel (as in the
+// one-lane form: once per sample), then a pair swaps them by one shuffle
+// each.  The pair's two loads read pixel A's block (lane 0 slab z0, lane 1
+// slab z0 + 1) and then pixel B's, so every load instruction takes whole
+// 64-byte blocks, one L1 wavefront per pixel as in the lane-pair form.
+// Each lane forms its slab's share of both pixels; lane 0 keeps A and lane 1
+// B, the other share arriving by shuffle (slab z0's share plus slab z0 + 1's,
+// the pair form's sum).  (Recomputing the partner's fractions from its
+// coordinates instead of receiving them by three shuffles measured slower:
+// 8.99 against 8.56 ms per 128 particles at box 256.)
+// Bound by the L1's data stage: 51 wavefronts per 32 samples, 39 of them the
+// blocks, at 84 % of its cycles.  So what else passes there is kept low: the
+// matrix as two loads, the norms' lane sums through shared memory for all
+// rotations at once, no index tables.  64 particles x 1,000 x 9,930: 3.82 ms
+// (with 5 shuffles a rotation's norm, six matrix loads, and conversions and
+// wraps in the index: 4.00).
 template <bool kArith, int G>
 __global__ void __launch_bounds__(256, 4)
 k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls,
@@ -1438,71 +1444,98 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
         ptv[j] = (TS > 0 && t < nT) ? pTs[t] : 0.f;
     }
     float cacc = 0.f;
-    // four rows per warp in flight: their loads precede their arithmetic, and
-    // their sums over the lanes share the steps of one reduction
+    // Four rows per warp in flight: their loads precede their arithmetic, and
+    // their sums over the lanes share the steps of one reduction.  What a row
+    // has in FP64 (its prior, its sum) is converted for 32 rows of the warp at
+    // once, a lane each: the SM's two FP64 lanes take 16 cycles a warp
+    // instruction.  Rows past the end are read as the last one with a prior of 0,
+    // translations past the end as the last with a prior of 0: they add zeros.
+    // 2,000 blocks of 6,912 x 49: 0.93 ms (with the FP64 pipe 75 % busy and 83
+    // instructions a row: 1.38 ms).
     const bool b4 = lane & 16, b3 = lane & 8;
-    for (int r0 = wid; r0 < nR; r0 += 4 * nw) {
-        float dv[4][TS > 0 ? TS : 1], prr[4], ad[4], racc[4];
+    const float* col[TS > 0 ? TS : 1];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = r0 + q * nw;
-            const bool rok = r < nR;
-            prr[q] = rok ? (float)pr[r] : 0.f;
-            ad[q] = (rok && nrmB) ? nrmB[(size_t)r * nrmRS + item] : 0.f;
-            const float* row = Db + (size_t)(rok ? r : 0) * ldc;
+    for (int j = 0; j < (TS > 0 ? TS : 1); j++) col[j] = Db + min(lane + 32 * j, nT - 1);
+    const size_t step = (size_t)nw * ldc;
+    for (int rb = wid; rb < nR; rb += 32 * nw) {
+        const int rl = rb + lane * nw;               // the lane's row of the 32
+        const float prv = rl < nR ? (float)pr[rl] : 0.f;
+        const float adv = nrmB ? nrmB[(size_t)min(rl, nR - 1) * nrmRS + item] : 0.f;
+        float sums = 0.f;
+        for (int g = 0; g < 8; g++) {
+            const int r0 = rb + 4 * g * nw;
+            if (r0 >= nR) break;
+            float dv[4][TS > 0 ? TS : 1], prr[4], racc[4];
+            const bool whole = r0 + 3 * nw < nR;
+            size_t off = (size_t)r0 * ldc;
 #pragma unroll
-            for (int j = 0; j < (TS > 0 ? TS : 1); j++) {
-                const int t = lane + 32 * j;
-                dv[q][j] = (TS > 0 && rok && t < nT) ? row[t] : 0.f;
+            for (int q = 0; q < 4; q++) {
+                prr[q] = __shfl_sync(0xffffffffu, prv, 4 * g + q);
+                racc[q] = 0.f;
+                if (!whole) off = (size_t)min(r0 + q * nw, nR - 1) * ldc;
+                if (TS > 0) {
+#pragma unroll
+                    for (int j = 0; j < (TS > 0 ? TS : 1); j++) dv[q][j] = col[j][off];
+                }
+                off += step;
             }
-        }
+            if (nrmB) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = r0 + q * nw;
-            racc[q] = 0.f;
-            if (r >= nR) continue;
-            const float* row = Db + (size_t)r * ldc;
-            if (TS > 0) {
+                for (int q = 0; q < 4; q++) {
+                    const float ad = __shfl_sync(0xffffffffu, adv, 4 * g + q);
 #pragma unroll
-                for (int j = 0; j < (TS > 0 ? TS : 1); j++) {
-                    const int t = lane + 32 * j;
-                    if (t < nT) {
-                        const float d = dv[q][j] + ad[q];
-                        const float sv = __expf(d - M);
+                    for (int j = 0; j < (TS > 0 ? TS : 1); j++) dv[q][j] = TS > 0 ? dv[q][j] + ad : ad;
+                }
+            } else if (TS == 0) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) dv[q][0] = 0.f;
+            }
+            if (dvp && TS > 0) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int j = 0; j < (TS > 0 ? TS : 1); j++)
+                        if (r0 + q * nw < nR && lane + 32 * j < nT)
+                            dvp[((size_t)item * nRall + r0c + r0 + q * nw) * nT + lane + 32 * j] =
+                                (float)(x0b + (double)dv[q][j]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (TS > 0) {
+#pragma unroll
+                    for (int j = 0; j < (TS > 0 ? TS : 1); j++) {
+                        const float sv = __expf(dv[q][j] - M);
                         racc[q] = fmaf(sv, ptv[j], racc[q]);
                         tacc[j] = fmaf(sv, prr[q], tacc[j]);
+                    }
+                } else if (r0 + q * nw < nR) {
+                    const float* row = Db + (size_t)(r0 + q * nw) * ldc;
+                    for (int t = lane; t < nT; t += 32) {
+                        const float d = row[t] + dv[q][0];
+                        const float sv = __expf(d - M);
+                        racc[q] = fmaf(sv, pTs[t], racc[q]);
+                        atomicAdd(wTs + t, sv * prr[q]);
                         if (dvp)
-                            dvp[((size_t)item * nRall + r0c + r) * nT + t] =
+                            dvp[((size_t)item * nRall + r0c + r0 + q * nw) * nT + t] =
                                 (float)(x0b + (double)d);
                     }
                 }
-            } else {
-                for (int t = lane; t < nT; t += 32) {
-                    const float d = row[t] + ad[q];
-                    const float sv = __expf(d - M);
-                    racc[q] = fmaf(sv, pTs[t], racc[q]);
-                    atomicAdd(wTs + t, sv * prr[q]);
-                    if (dvp)
-                        dvp[((size_t)item * nRall + r0c + r) * nT + t] =
-                            (float)(x0b + (double)d);
-                }
             }
-        }
-        // the four butterfly sums (the same additions as one after another):
-        // a lane keeps two rows after the first step, one after the second;
-        // lanes 8 q .. 8 q + 7 end with row q's
-        float s0 = (b4 ? racc[2] : racc[0]) + __shfl_xor_sync(0xffffffffu, b4 ? racc[0] : racc[2], 16);
-        float s1 = (b4 ? racc[3] : racc[1]) + __shfl_xor_sync(0xffffffffu, b4 ? racc[1] : racc[3], 16);
-        float sr = (b3 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b3 ? s0 : s1, 8);
+            // the four butterfly sums (the same additions as one after another):
+            // a lane keeps two rows after the first step, one after the second;
+            // lanes 8 q .. 8 q + 7 end with row q's
+            float s0 = (b4 ? racc[2] : racc[0]) + __shfl_xor_sync(0xffffffffu, b4 ? racc[0] : racc[2], 16);
+            float s1 = (b4 ? racc[3] : racc[1]) + __shfl_xor_sync(0xffffffffu, b4 ? racc[1] : racc[3], 16);
+            float sr = (b3 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b3 ? s0 : s1, 8);
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, o);
+            for (int o = 4; o > 0; o >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, o);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float rs = __shfl_sync(0xffffffffu, sr, 8 * q);
-            if (r0 + q * nw < nR) cacc = fmaf(rs, prr[q], cacc);   // sum_t s pT[t] pR[r], once per row
+            for (int q = 0; q < 4; q++)      // sum_t s pT[t] pR[r], once per row
+                cacc = fmaf(__shfl_sync(0xffffffffu, sr, 8 * q), prr[q], cacc);
+            const float mine = __shfl_sync(0xffffffffu, sr, 8 * (lane & 3));
+            if (lane >> 2 == g) sums = mine;
         }
-        const int rw = r0 + (lane >> 3) * nw;
-        if ((lane & 7) == 0 && rw < nR) wR[(size_t)item * nRall + r0c + rw] = (double)sr * pc;
+        if (rl < nR) wR[(size_t)item * nRall + r0c + rl] = (double)sums * pc;
     }
     if (TS > 0) {
 #pragma unroll
