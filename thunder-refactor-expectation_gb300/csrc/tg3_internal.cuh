@@ -67,10 +67,10 @@ __device__ __forceinline__ void fill_brick_tables(int vdim, int* tx, int* ty, in
     const int nx = vdim / 2 + 1;
     const int nxc = cubes_x(vdim), nyc = cubes_yz(vdim);
     for (int j = threadIdx.x; j < nx; j += blockDim.x)
-        tx[j] = (j >> 5) * 32768 + ((j >> 3) & 3) * 512 + (j & 7);
+        tx[j] = (j >> 5) * 32768 + (j & 31);
     for (int j = threadIdx.x; j < vdim; j += blockDim.x) {
-        ty[j] = (j >> 5) * nxc * 32768 + ((j >> 3) & 3) * 2048 + (j & 7) * 8;
-        tz[j] = (j >> 5) * nyc * nxc * 32768 + ((j >> 3) & 3) * 8192 + (j & 7) * 64;
+        ty[j] = (j >> 5) * nxc * 32768 + (j & 31) * 32;
+        tz[j] = (j >> 5) * nyc * nxc * 32768 + (j & 31) * 1024;
     }
 }
 

@@ -171,18 +171,15 @@ __global__ void k_ctf(const float* __restrict__ attr, int nImg, float px, int id
 
 // Placement of the corner block of voxel (z, y, x), z and y counted from the
 // lowest coordinate -vdim / 2 (so that a sample's index needs no wrap): the
-// volume is cut into
-// cubes of 32^3 voxels (32768 blocks = 2 MB, one large page each, cubes in
-// z, y, x order), each cube into 4^3 bricks of 8^3 voxels, voxels x-fastest
-// within a brick.  A projection's samples within one pixel band then touch a
-// few hundred pages instead of one page per z plane of the band, which in
-// the plain [z][y][x] order left the gather translation-bound.
+// volume is cut into cubes of 32^3 voxels (32768 blocks = 2 MB, one large page
+// each, cubes in z, y, x order), voxels x-fastest within a cube.  A projection's
+// samples within one pixel band then touch a few hundred pages instead of one
+// page per z plane of the band, which in the plain [z][y][x] order left the
+// gather translation-bound.
 __device__ __forceinline__ size_t brick_index(int x, int y, int z, int nxc, int nyc)
 {
     const size_t cube = ((size_t)(z >> 5) * nyc + (y >> 5)) * nxc + (x >> 5);
-    const int brick = (((z >> 3) & 3) * 4 + ((y >> 3) & 3)) * 4 + ((x >> 3) & 3);
-    const int v = ((z & 7) * 8 + (y & 7)) * 8 + (x & 7);
-    return (cube * 64 + brick) * 512 + v;
+    return cube * 32768 + ((z & 31) * 32 + (y & 31)) * 32 + (x & 31);
 }
 
 
@@ -478,8 +475,7 @@ k_project_lane(float4* const* __restrict__ volTable, const int* __restrict__ cls
             if (kArith) {
                 const int yy = y0 + half, zz = z0 + half;
                 blk = (unsigned)((((zz >> 5) * nyc + (yy >> 5)) * nxc + (x0 >> 5)) * 32768
-                                 + ((((zz >> 3) & 3) * 4 + ((yy >> 3) & 3)) * 4 + ((x0 >> 3) & 3)) * 512
-                                 + ((zz & 7) * 8 + (yy & 7)) * 8 + (x0 & 7));
+                                 + ((zz & 31) * 32 + (yy & 31)) * 32 + (x0 & 31));
             } else {
                 blk = (unsigned)(tx[x0] + ty[y0 + half] + tz[z0 + half]);
             }
@@ -540,58 +536,106 @@ k_project_lane(float4* const* __restrict__ volTable, const int* __restrict__ cls
     }
 }
 
-// Block index and fractions of a sample, without tables and conversions: the
-// floor comes out of an addition rounded down (x + 1.5 2^23 has the integer part
-// of x in its low bits), the index fields (brick_index) out of shifted copies
-// of those bits, x = a + 8 b + 32 c -> a + 512 b + 32768 c and so on, with all
-// offsets in one constant.  A coordinate outside the volume (not a number) is
-// held to the blocks there are.
+// Two FP32 values in a 64-bit register, and the two-wide operations on them.
+__device__ __forceinline__ uint64_t pack2(float x, float y)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mad2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
+{
+    return mad2(b, pack2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ uint64_t add2_down(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Block indexes and fractions of two samples, without tables and conversions:
+// the floor comes out of an addition rounded down (x + 1.5 2^23 has the integer
+// part of x in its low bits), the index (brick_index) out of shifted copies of
+// those bits, x = a + 32 b -> a + 32768 b and so on, with all offsets in one
+// constant.  A coordinate outside the volume (not a number) is held to the
+// blocks there are.
 struct BrickIndex {
     unsigned yc, zc, offset, last;
     float yMagic;
     __device__ __forceinline__ explicit BrickIndex(int vdim)
     {
         const unsigned nxc = cubes_x(vdim), nyc = cubes_yz(vdim), bias = 0x4b400000u;
-        yc = nxc * 32768u - 8192u;
+        yc = nxc * 32768u - 1024u;
         zc = nxc * nyc * 32768u - 32768u;
         yMagic = 12582912.f + (float)(vdim / 2);
         last = nxc * nyc * nyc * 32768u - 1u;
-        offset = 0u - (bias + 504u * (bias >> 3) + 30720u * (bias >> 5)) -
-                 (8u * bias + 1984u * (bias >> 3) + yc * (bias >> 5)) -
-                 (64u * bias + 7680u * (bias >> 3) + zc * (bias >> 5));
+        offset = 0u - (bias + 32736u * (bias >> 5)) - (32u * bias + yc * (bias >> 5)) -
+                 (1024u * bias + zc * (bias >> 5));
     }
-    __device__ __forceinline__ unsigned operator()(float x, float y, float z, float (&f)[3]) const
+    __device__ __forceinline__ void operator()(const uint64_t (&v)[3], uint64_t (&f)[3],
+                                               unsigned (&b)[2]) const
     {
-        const float tx = __fadd_rd(x, 12582912.f), ty = __fadd_rd(y, yMagic),
-                    tz = __fadd_rd(z, yMagic);
-        f[0] = x - (tx - 12582912.f);
-        f[1] = y - (ty - yMagic);
-        f[2] = z - (tz - yMagic);
-        const unsigned bx = __float_as_uint(tx), by = __float_as_uint(ty), bz = __float_as_uint(tz);
-        const unsigned b = offset + bx + 504u * (bx >> 3) + 30720u * (bx >> 5) + 8u * by +
-                           1984u * (by >> 3) + yc * (by >> 5) + 64u * bz + 7680u * (bz >> 3) +
-                           zc * (bz >> 5);
-        return min(b, last);
+        const float magic[3] = {12582912.f, yMagic, yMagic};
+        unsigned n[3][2];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const uint64_t t = add2_down(v[k], pack2(magic[k], magic[k]));
+            f[k] = sub2(v[k], add2(t, pack2(-magic[k], -magic[k])));
+            n[k][0] = (unsigned)t;
+            n[k][1] = (unsigned)(t >> 32);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const unsigned x = n[0][i], y = n[1][i], z = n[2][i];
+            b[i] = min(offset + x + 32736u * (x >> 5) + 32u * y + yc * (y >> 5) + 1024u * z +
+                           zc * (z >> 5),
+                       last);
+        }
     }
 };
 
-// Lane pairs that share loads but not the coordinate work (forms 3 and 4).
-// Every lane finds the block index and fractions of its own pixel (as in the
-// one-lane form: once per sample), then a pair swaps them by one shuffle
-// each.  The pair's two loads read pixel A's block (lane 0 slab z0, lane 1
-// slab z0 + 1) and then pixel B's, so every load instruction takes whole
-// 64-byte blocks, one L1 wavefront per pixel as in the lane-pair form.
-// Each lane forms its slab's share of both pixels; lane 0 keeps A and lane 1
-// B, the other share arriving by shuffle (slab z0's share plus slab z0 + 1's,
-// the pair form's sum).  (Recomputing the partner's fractions from its
-// coordinates instead of receiving them by three shuffles measured slower:
-// 8.99 against 8.56 ms per 128 particles at box 256.)
-// Bound by the L1's data stage: 51 wavefronts per 32 samples, 39 of them the
-// blocks, at 84 % of its cycles.  So what else passes there is kept low: the
-// matrix as two loads, the norms' lane sums through shared memory for all
-// rotations at once, no index tables.  64 particles x 1,000 x 9,930: 3.82 ms
-// (with 5 shuffles a rotation's norm, six matrix loads, and conversions and
-// wraps in the index: 4.00).
+// Lane pairs that share loads (forms 3 and 4).  The pair's two loads read pixel
+// A's block (the even lane slab z0, the odd lane slab z0 + 1) and then pixel B's,
+// so every load instruction takes whole 64-byte blocks, one L1 wavefront per
+// pixel as in the lane-pair form.  Each lane forms its slab's share of both
+// pixels; the even lane keeps A and the odd one B, the other share arriving by
+// shuffle (slab z0's share plus slab z0 + 1's, the pair form's sum).
+// Coordinates, fractions and weights of A and B are formed together, two-wide.
+// In form 4 (kArith) both lanes form them for both pixels; in form 3 a lane
+// finds its own pixel's block by table and fractions, and the pair swaps them.
+// Form 4 is bound by the L1's data stage and the issue slots about alike: 47
+// wavefronts per 32 samples, 39 of them the blocks (80 % of its cycles), 176
+// instructions (72 %).  So the matrix comes as two loads, the norms' lane sums go
+// through shared memory for all rotations at once, and the index needs neither
+// tables nor conversions nor exchange.  64 particles x 1,000 x 9,930: 3.73 ms;
+// with four shuffles for the exchange 3.82; with five more a norm, six matrix
+// loads, and conversions, wraps and 8^3 bricks in the index 4.00.
 template <bool kArith, int G>
 __global__ void __launch_bounds__(256, 4)
 k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls,
@@ -660,13 +704,18 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
     const float fpf = (float)pf;
     const float* sg = sigRcp ? sigRcp + (size_t)l * K : nullptr;
     const float* cf = ctf ? ctf + (size_t)l * K : nullptr;
-    float pa[kLaneU], pb[kLaneU], w2[kLaneU];
+    // own pixels' weights; the coordinates of the pair's pixels A and B (of the own
+    // one, twice, with the table)
+    uint64_t pa[kLaneU], pb[kLaneU];
+    float w2[kLaneU];
 #pragma unroll
     for (int u = 0; u < kLaneU; u++) {
         const int p = pBase + u * 256;
         const int q = p < K ? p : 0;
-        pa[u] = (float)iCol[q] * fpf;
-        pb[u] = (float)iRow[q] * fpf;
+        const float a = (float)iCol[q] * fpf, b = (float)iRow[q] * fpf;
+        const float a1 = __shfl_xor_sync(0xffffffffu, a, 1), b1 = __shfl_xor_sync(0xffffffffu, b, 1);
+        pa[u] = !kArith ? pack2(a, a) : h ? pack2(a1, a) : pack2(a, a1);
+        pb[u] = !kArith ? pack2(b, b) : h ? pack2(b1, b) : pack2(b, b1);
         w2[u] = (nrmPart && p < K) ? sg[q] * cf[q] * cf[q] : 0.f;
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -675,28 +724,40 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
         const float4 m01 = *reinterpret_cast<const float4*>(m[i]);
         const float2 m2 = *reinterpret_cast<const float2*>(m[i] + 4);
         float acc = 0.f;
-        float fo[kLaneU][3], fp[kLaneU][3];   // own and partner fractions
+        uint64_t f[kLaneU][3];                // fractions of A and B
+        unsigned blk[kLaneU][2];              // block index of A and B
         bool cj[kLaneU];
-        unsigned bo[kLaneU], bp[kLaneU];      // own and partner block index
 #pragma unroll
         for (int u = 0; u < kLaneU; u++) {
-            float x = m01.x * pa[u] + m01.y * pb[u];
-            float y = m01.z * pa[u] + m01.w * pb[u];
-            float z = m2.x * pa[u] + m2.y * pb[u];
-            cj[u] = x < 0.f;
-            if (cj[u]) { x = -x; y = -y; z = -z; }
-            if (kArith) {
-                bo[u] = bi(x, y, z, fo[u]);
-            } else {
-                const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
-                fo[u][0] = x - xf;
-                fo[u][1] = y - yf;
-                fo[u][2] = z - zf;
-                bo[u] = (unsigned)(tx[(int)xf] + ty[(int)yf + half] + tz[(int)zf + half]);
-            }
-            bp[u] = __shfl_xor_sync(0xffffffffu, bo[u], 1);
+            uint64_t v[3] = {mad2(pack2(m01.x, m01.x), pa[u], mul2(pack2(m01.y, m01.y), pb[u])),
+                             mad2(pack2(m01.z, m01.z), pa[u], mul2(pack2(m01.w, m01.w), pb[u])),
+                             mad2(pack2(m2.x, m2.x), pa[u], mul2(pack2(m2.y, m2.y), pb[u]))};
+            const float2 x = unpack2(v[0]);
+            cj[u] = (kArith && h ? x.y : x.x) < 0.f;
+            const uint64_t sign = pack2(x.x < 0.f ? -1.f : 1.f, x.y < 0.f ? -1.f : 1.f);
 #pragma unroll
-            for (int k = 0; k < 3; k++) fp[u][k] = __shfl_xor_sync(0xffffffffu, fo[u][k], 1);
+            for (int k = 0; k < 3; k++) v[k] = mul2(v[k], sign);
+            if (kArith) {
+                bi(v, f[u], blk[u]);
+            } else {
+                float o[3];
+                int n[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const float c = unpack2(v[k]).x, fl = floorf(c);
+                    o[k] = c - fl;
+                    n[k] = (int)fl;
+                }
+                const unsigned own = (unsigned)(tx[n[0]] + ty[n[1] + half] + tz[n[2] + half]);
+                const unsigned other = __shfl_xor_sync(0xffffffffu, own, 1);
+                blk[u][0] = h ? other : own;
+                blk[u][1] = h ? own : other;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const float p = __shfl_xor_sync(0xffffffffu, o[k], 1);
+                    f[u][k] = h ? pack2(p, o[k]) : pack2(o[k], p);
+                }
+            }
         }
         // slab h of pixel A (the even lane's) then of pixel B (the odd lane's)
         float4 c[kLaneU][4];
@@ -704,8 +765,7 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
         for (int u = 0; u < kLaneU; u++)
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const unsigned b = (k == 0) == (h == 0) ? bo[u] : bp[u];
-                const float4* e = vol + 4 * (size_t)b + 2 * h;
+                const float4* e = vol + 4 * (size_t)blk[u][k] + 2 * h;
                 asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                     : "=f"(c[u][2 * k].x), "=f"(c[u][2 * k].y), "=f"(c[u][2 * k].z),
                       "=f"(c[u][2 * k].w), "=f"(c[u][2 * k + 1].x), "=f"(c[u][2 * k + 1].y),
@@ -714,21 +774,23 @@ k_project_xchg(float4* const* __restrict__ volTable, const int* __restrict__ cls
             }
 #pragma unroll
         for (int u = 0; u < kLaneU; u++) {
+            const uint64_t one = pack2(1.f, 1.f);
+            const uint64_t wx0 = sub2(one, f[u][0]), wx1 = f[u][0];
+            const uint64_t wz = h ? f[u][2] : sub2(one, f[u][2]);
+            const uint64_t wy0 = mul2(sub2(one, f[u][1]), wz), wy1 = mul2(f[u][1], wz);
+            const uint64_t w00 = mul2(wx0, wy0), w10 = mul2(wx1, wy0), w01 = mul2(wx0, wy1),
+                           w11 = mul2(wx1, wy1);
             float sr[2], si[2];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const bool own = (k == 0) == (h == 0);
-                const float fx = own ? fo[u][0] : fp[u][0];
-                const float fy = own ? fo[u][1] : fp[u][1];
-                const float fz = own ? fo[u][2] : fp[u][2];
-                const float wz = h ? fz : 1.f - fz;
-                const float wx0 = 1.f - fx, wx1 = fx;
-                const float wy0 = (1.f - fy) * wz, wy1 = fy * wz;
+                const float2 p = unpack2(w00), q = unpack2(w10), r = unpack2(w01), t = unpack2(w11);
+                const float v00 = k ? p.y : p.x, v10 = k ? q.y : q.x, v01 = k ? r.y : r.x,
+                            v11 = k ? t.y : t.x;
                 const float4 a = c[u][2 * k], b = c[u][2 * k + 1];
-                float re = a.x * (wx0 * wy0) + a.z * (wx1 * wy0);
-                float im = a.y * (wx0 * wy0) + a.w * (wx1 * wy0);
-                re += b.x * (wx0 * wy1) + b.z * (wx1 * wy1);
-                im += b.y * (wx0 * wy1) + b.w * (wx1 * wy1);
+                float re = a.x * v00 + a.z * v10;
+                float im = a.y * v00 + a.w * v10;
+                re += b.x * v01 + b.z * v11;
+                im += b.y * v01 + b.w * v11;
                 sr[k] = re;
                 si[k] = im;
             }
@@ -1178,20 +1240,6 @@ __global__ void k_x0(const float2* __restrict__ dat, const float* __restrict__ s
 // The staged tiles are transposed, [k][row], with row XOR f(k): f spreads the
 // BK / 4 float4 columns that a warp stores together over the banks (no
 // conflict at any BK) and moves whole float4 groups, so the reads stay vectors.
-__device__ __forceinline__ uint64_t pack2(float x, float y)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-
-__device__ __forceinline__ float2 unpack2(uint64_t v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
 __device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b)
 {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
