@@ -974,13 +974,13 @@ static int insert_draws(tg3_ctx* c, int nDraws, int drawsPerImage, const float* 
         return TG3_OK;
     }
     float* params = static_cast<float*>(
-        ws_get(c, WS_INSERT, (size_t)nDraws * 16 * sizeof(float), &st));
+        ws_get(c, WS_INSERT, insert_param_bytes(nDraws, c->px.K), &st));
     if (st) return st;
     TG3_CUDA(launch_insert(c->ins.acc, c->ins.vdim, kernel, c->ins.tab, c->ins.tabNz,
                            c->ins.tabInvStep, nDraws, drawsPerImage,
                            reinterpret_cast<const float2*>(dat), ctf, quat, trans, offset, w,
                            c->px.iCol, c->px.iRow, c->px.K, c->ins.pf, c->px.idim, O3D,
-                           counter, params, c->stream, ctfRows, nC));
+                           counter, params, c->stream, c->px.maxRadius, ctfRows, nC));
     return TG3_OK;
 }
 

@@ -368,8 +368,11 @@ cudaError_t launch_resample(int nP, int n, const double* u, const double* w,
                             cudaStream_t st,
                             const int* nPer = nullptr);
 // k_insert_draws (one thread per draw: parameters into params, 16 floats
-// per draw, and the O3D / counter bookkeeping), then k_insert: CTA (share
-// of the pixels, draw); draw d uses image d / drawsPerImage.
+// per draw, a work counter and the pixels' order, and the O3D / counter
+// bookkeeping; maxRadius: of the pixels), then
+// k_insert_mkb (persistent) or k_insert (trilinear; CTA (share of the pixels,
+// draw)); draw d uses image d / drawsPerImage.
+size_t insert_param_bytes(int nDraws, int K);
 cudaError_t launch_insert(float4* acc, int vdim, int kernel, const float* tab,
                           int tabNz, float tabInvStep, int nDraws,
                           int drawsPerImage, const float2* dat,
@@ -377,7 +380,7 @@ cudaError_t launch_insert(float4* acc, int vdim, int kernel, const float* tab,
                           const double* trans, const double* offset,
                           const float* w, const int* iCol, const int* iRow,
                           int K, int pf, int idim, double* O3D, int* counter,
-                          float* params, cudaStream_t st, int ctfRows = 0,
+                          float* params, cudaStream_t st, double maxRadius, int ctfRows = 0,
                           const int* nC = nullptr);
 // MKB insertion by gather: per chunk of draws, k_insert_stage (tiles x
 // draws) fills the draws' dense pixel grids from the cell map cellPix,
