@@ -580,7 +580,7 @@ static int local_phase(tg3_ctx* c, const int* bankIdx, int nP, int nR, int nT, c
             }
             TG3_CUDA(launch_gemm_bank_bf16x3(c->bank, c->px.gen, bankIdx, cls, nP, nR, A, nT, Kp,
                                              K, sigRcp, ctf, D, -2.0f, c->d_flag, s,
-                                             c->bankGather == 2, order, c->bankShape));
+                                             c->bankGather == 2, order, c->bankShape, P));
         }
         {
             StageTimer tm(c, TG3_STAGE_WEIGHTS);

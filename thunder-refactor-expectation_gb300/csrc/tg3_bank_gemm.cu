@@ -61,6 +61,7 @@ struct BgParams {
     const int* order;              // [nP] particle of each grid row (null: identity)
     const float* sigRcp;           // [nP][K]
     const float* ctf;              // [nP][K]
+    const float* wn;               // [nP][Kd / 2] sigRcp ctf^2, zeros past K (cp.async form)
     float* C;                      // [nP][nR][nT]
     float alpha;
     int* flag;
@@ -336,15 +337,23 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src)
                  : "memory");
 }
 
-// CP_PW gather warps (eight by default, 0 - 7), then the B-tile TMA warp
-// (CP_PW) and the MMA warp (CP_PW + 1, which also holds the tensor memory);
-// warps 0 - 3 run the epilogue.
+// CP_PW gather warps (eight by default), which also sum the norms, or (NW > 0) NW
+// norm warps first; then the B-tile TMA warp and the MMA warp, which also holds
+// the tensor memory; warps 0 - 3 run the epilogue.
+//
+// With norm warps a stage is free when they have read it too.  A K block's time is
+// neither HBM's nor L2's (rows that all lie in L2 take as long, and so do other
+// lags): it is what the warps execute one after another, and shared memory, of
+// which the copies, the norms' reads and the tensor core's take about 1,200 of
+// 1,670 cycles.  1,000 particles x 256 rows x 25: 3.51 ms; 16 warps doing both
+// 3.74 (with scalar weights and divisions by the number of stages 4.31), 8 warps
+// 4.08.
 //
 // BK is the K block: 64 bf16 (128-byte rows, 128-byte swizzle) or 32
 // (64-byte rows, 64-byte swizzle: half the bytes a stage, so more stages, or
 // two CTAs an SM with MINB = 2).  A row's chunk of a K block is BK / 8
 // 16-byte pieces, one per lane of a row group; a thread copies CP_RPT rows.
-constexpr int cp_threads(int pw) { return (pw + 2) * 32; }
+constexpr int cp_threads(int pw, int nw) { return (pw + nw + 2) * 32; }
 
 template <int BK>
 __device__ __forceinline__ uint64_t bank_desc(uint32_t saddr)
@@ -362,14 +371,17 @@ __device__ __forceinline__ int bank_phys(int r, int q)
                     : (r >> 3) * 512 + (r & 7) * 64 + ((q ^ ((r >> 1) & 3)) << 4);
 }
 
-template <int S, int BK, int MINB, int CP_PW = 8>
-__global__ void __launch_bounds__(cp_threads(CP_PW), MINB)
+template <int S, int BK, int MINB, int CP_PW = 8, int NW = 0>
+__global__ void __launch_bounds__(cp_threads(CP_PW, NW), MINB)
 k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
                const __grid_constant__ CUtensorMap tmBl, const BgParams p)
 {
     constexpr int QPR = BK / 8;                          // 16-byte chunks per row
     constexpr int CP_RPT = BG_M * QPR / (CP_PW * 32);     // rows per gather thread
     constexpr int RSTRIDE = CP_PW * 32 / QPR;             // rows between a thread's rows
+    constexpr int NPW = NW ? NW : CP_PW;                  // warps that sum norms: 0 .. NPW - 1
+    constexpr int NRPT = BG_M * QPR / (NPW * 32), NSTRIDE = NPW * 32 / QPR;
+    constexpr int TMA_WARP = CP_PW + NW;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -408,13 +420,13 @@ k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
     if (threadIdx.x == BG_M) {
         for (int s = 0; s < S; s++) {
             mbar_init(full + s, CP_PW + 1);
-            mbar_init(empty + s, 1);
+            mbar_init(empty + s, 1 + NW);
         }
         mbar_init(accum, 1);
         *abortFlag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == CP_PW + 1) {
+    if (warp == TMA_WARP + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmemSlot)),
                      "r"(p.tmemCols)
@@ -427,9 +439,69 @@ k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
     const uint32_t tmem = *tmemSlot;
 
     int issuedTma = 0, issuedMma = 0;
-    if (warp < CP_PW) {
-        // ---------------- A tiles and the rows' norms
-        const int t = threadIdx.x;
+    // the norms: thread t takes chunk t % QPR of the rows t / QPR, NSTRIDE apart
+    const int nq = threadIdx.x % QPR, ng = threadIdx.x / QPR;
+    float nS[NRPT], nC[NRPT];
+#pragma unroll
+    for (int i = 0; i < NRPT; i++) nS[i] = nC[i] = 0.f;
+    const float4* wn = reinterpret_cast<const float4*>(p.wn + (size_t)item * (p.Kd / 2)) + nq;
+    auto norms = [&](const uint8_t* st, const float4& w4) {
+        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+        for (int i = 0; i < NRPT; i++) {
+            const int at = bank_phys<BK>(ng + NSTRIDE * i, nq);
+            const uint4 h = *reinterpret_cast<const uint4*>(st + at);
+            const uint4 lo = *reinterpret_cast<const uint4*>(st + aBytes + at);
+            const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, lw[4] = {lo.x, lo.y, lo.z, lo.w};
+            float part = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float2 hf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hw[c]));
+                const float2 lf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&lw[c]));
+                const float re = hf.x + lf.x, im = hf.y + lf.y;
+                part = fmaf(w[c], re * re + im * im, part);
+            }
+            kahan_add(nS[i], nC[i], part);
+        }
+    };
+    // the rows' norms: the QPR lanes of a row group hold partials
+    auto store_norms = [&]() {
+#pragma unroll
+        for (int i = 0; i < NRPT; i++) {
+            float v = nS[i] - nC[i];
+#pragma unroll
+            for (int o = 1; o < QPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (nq == 0) nrmRow[ng + NSTRIDE * i] = v;
+        }
+    };
+    if (NW && warp < NW) {
+        // ---------------- the rows' norms, a landed K block at a time
+        float4 w = __ldg(wn);
+        int s = 0, phase = 0;
+        for (int kb = 0; kb < nkb; kb++) {
+            const float4 wNext = __ldg(wn + (size_t)min(kb + 1, nkb - 1) * (BK / 8));
+            // every lane waits itself: the copies are other threads' writes
+            const bool ok = __all_sync(0xffffffffu, mbar_wait(full + s, phase, kWaitBudget));
+            if (!ok || *(volatile int*)abortFlag) {
+                if (lane == 0) {
+                    atomicOr(p.flag, 4);
+                    *(volatile int*)abortFlag = 1;
+                }
+                break;
+            }
+            norms(smem + s * stageBytes, w);
+            w = wNext;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + s);
+            if (++s == S) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
+        store_norms();
+    } else if (warp < TMA_WARP) {
+        // ---------------- A tiles (and, without norm warps, the rows' norms)
+        const int t = threadIdx.x - NW * 32;
         const int g = t / QPR, q = t % QPR;                // row group, 16-byte chunk
         const __nv_bfloat16* bh = banks.hi[k];
         const __nv_bfloat16* bl = banks.lo[k];
@@ -444,28 +516,14 @@ k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
             srcL[i] = bl + off;
             phys[i] = bank_phys<BK>(r, q);
         }
-        const float* sg = p.sigRcp + (size_t)item * p.K;
-        const float* cf = p.ctf + (size_t)item * p.K;
-        float nS[CP_RPT], nC[CP_RPT];
-#pragma unroll
-        for (int i = 0; i < CP_RPT; i++) nS[i] = nC[i] = 0.f;
-        // the weights sigRcp ctf^2 of this lane's 4 pixels, one K block ahead
-        auto weights = [&](int kd, float* w) {
-            const int px0 = kd * (BK / 2) + q * 4;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int px = px0 + c;
-                const float cc = px < p.K ? __ldg(cf + px) : 0.f;
-                w[c] = px < p.K ? __ldg(sg + px) * cc * cc : 0.f;
-            }
-        };
-        float wCur[4], wNext[4];
-        weights(0, wCur);
+        // the weights of this lane's 4 pixels, one K block ahead
+        float4 wNext = NW ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(wn);
         constexpr int LAG = S > 3 ? S - 3 : 0;
+        // stage and use of it of the block being copied, stage of the one that
+        // has landed
+        int s = 0, round = 0, sd = 0;
         for (int kb = 0; kb < nkb + LAG; kb++) {
             if (kb < nkb) {
-                const int s = kb % S;
-                const int round = kb / S;
                 if (round > 0) {
                     bool ok = lane != 0 || mbar_wait(empty + s, (round - 1) & 1, kWaitBudget);
                     ok = __all_sync(0xffffffffu, ok);
@@ -478,11 +536,16 @@ k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
                     }
                 }
                 uint8_t* st = smem + s * stageBytes;
-                const size_t o = (size_t)kb * BK;
 #pragma unroll
                 for (int i = 0; i < CP_RPT; i++) {
-                    cp_async16(st + phys[i], srcH[i] + o);
-                    cp_async16(st + aBytes + phys[i], srcL[i] + o);
+                    cp_async16(st + phys[i], srcH[i]);
+                    cp_async16(st + aBytes + phys[i], srcL[i]);
+                    srcH[i] += BK;
+                    srcL[i] += BK;
+                }
+                if (++s == S) {
+                    s = 0;
+                    round++;
                 }
             }
             // one group per iteration (empty at the tail), so that
@@ -490,46 +553,23 @@ k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
             asm volatile("cp.async.commit_group;" ::: "memory");
             const int kd = kb - LAG;
             if (kd < 0) continue;
-            if (kd + 1 < nkb) weights(kd + 1, wNext);
+            const float4 wCur = wNext;
+            if (!NW) wNext = __ldg(wn + (size_t)min(kd + 1, nkb - 1) * (BK / 8));
             asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
             // the copies (generic proxy) visible to the tensor cores' reads;
-            // the stage is handed over before this thread's norm reads of it
-            // (reads both, and only this thread rewrites its chunks, S blocks on)
+            // without norm warps the stage is handed over before this thread's
+            // norm reads of it (reads both, and only this thread rewrites its
+            // chunks, S blocks on)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(full + kd % S);
-            const uint8_t* st = smem + (kd % S) * stageBytes;
-#pragma unroll
-            for (int i = 0; i < CP_RPT; i++) {
-                const uint4 h = *reinterpret_cast<const uint4*>(st + phys[i]);
-                const uint4 lo = *reinterpret_cast<const uint4*>(st + aBytes + phys[i]);
-                const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, lw[4] = {lo.x, lo.y, lo.z, lo.w};
-                float part = 0.f;
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const float2 hf = __bfloat1622float2(
-                        *reinterpret_cast<const __nv_bfloat162*>(&hw[c]));
-                    const float2 lf = __bfloat1622float2(
-                        *reinterpret_cast<const __nv_bfloat162*>(&lw[c]));
-                    const float re = hf.x + lf.x, im = hf.y + lf.y;
-                    part = fmaf(wCur[c], re * re + im * im, part);
-                }
-                kahan_add(nS[i], nC[i], part);
-            }
-#pragma unroll
-            for (int c = 0; c < 4; c++) wCur[c] = wNext[c];
+            if (lane == 0) mbar_arrive(full + sd);
+            if (!NW) norms(smem + sd * stageBytes, wCur);
+            if (++sd == S) sd = 0;
         }
         // copies still in flight after an abort land before the CTA leaves
         asm volatile("cp.async.wait_all;" ::: "memory");
-        // the rows' norms: the QPR lanes of a row group hold partials
-#pragma unroll
-        for (int i = 0; i < CP_RPT; i++) {
-            float v = nS[i] - nC[i];
-#pragma unroll
-            for (int o = 1; o < QPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (q == 0) nrmRow[g + RSTRIDE * i] = v;
-        }
-    } else if (warp == CP_PW) {
+        if (!NW) store_norms();
+    } else if (warp == TMA_WARP) {
         // ---------------- B tiles (TMA)
         if (lane == 0) {
             for (int kb = 0; kb < nkb; kb++) {
@@ -610,21 +650,34 @@ k_gemm_bank_cp(const LdgRows banks, const __grid_constant__ CUtensorMap tmBh,
             for (int j = lane; j < p.nT; j += 32) cbase[(size_t)r * p.nT + j] = stage[rr * pitch + j];
         }
     }
-    if (aborted && warp == CP_PW && lane == 0) {
+    if (aborted && warp == TMA_WARP && lane == 0) {
         for (int kb = 0; kb < issuedTma; kb++) {
             const int s = kb % S;
             mbar_wait(full + s, (kb / S) & 1, kWaitBudget / 4);
         }
     }
-    if (aborted && warp == CP_PW + 1 && lane == 0 && issuedMma > 0)
+    if (aborted && warp == TMA_WARP + 1 && lane == 0 && issuedMma > 0)
         mbar_wait(accum, 0, kWaitBudget / 4);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == CP_PW + 1) {
+    if (warp == TMA_WARP + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(p.tmemCols)
                      : "memory");
+    }
+}
+
+// wn[l][px] = sigRcp ctf^2, zeros for K <= px < Kh: the norm warps then load a
+// lane's four weights at once, where eight scalar loads and their bounds were a
+// fifth of what they execute.
+__global__ void k_bank_weights(const float* __restrict__ sigRcp, const float* __restrict__ ctf,
+                               int K, int Kh, float* __restrict__ wn)
+{
+    const size_t l = blockIdx.y;
+    for (int px = blockIdx.x * blockDim.x + threadIdx.x; px < Kh; px += gridDim.x * blockDim.x) {
+        const float cc = px < K ? ctf[l * K + px] : 0.f;
+        wn[l * Kh + px] = px < K ? sigRcp[l * K + px] * cc * cc : 0.f;
     }
 }
 
@@ -672,7 +725,7 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
                                     const int* cls, int nP, int nR, const void* B, int nT,
                                     int Kd, int K, const float* sigRcp, const float* ctf,
                                     float* C, float alpha, int* flag, cudaStream_t st,
-                                    bool tmaGather, int* order, int shape)
+                                    bool tmaGather, int* order, int shape, float* wn)
 {
     if (shape < 0 || shape > 3) return cudaErrorInvalidValue;
     if (nP <= 0 || nR <= 0 || nT <= 0 || nT > 256 || Kd <= 0 || Kd % BG_BK || nP > 65535)
@@ -728,6 +781,7 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
     }
     p.sigRcp = sigRcp;
     p.ctf = ctf;
+    p.wn = nullptr;
     p.C = C;
     p.alpha = alpha;
     p.flag = flag;
@@ -749,6 +803,9 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
         k_gemm_bank_bf16x3<<<grid, BG_THREADS, smem, st>>>(maps, mBh, mBl, p);
         return cudaGetLastError();
     }
+    if (!wn) return cudaErrorInvalidValue;
+    k_bank_weights<<<dim3((Kd / 2 + 1023) / 1024, nP), 256, 0, st>>>(sigRcp, ctf, K, Kd / 2, wn);
+    p.wn = wn;
     LdgRows rowsOf;
     for (int k = 0; k < kMaxClasses; k++) {
         const Bank& b = banks[maps.nB[k] ? k : first];
@@ -774,8 +831,8 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
         kern = S == 5 ? k_gemm_bank_cp<5, 64, 1> : S == 4 ? k_gemm_bank_cp<4, 64, 1>
              : S == 3 ? k_gemm_bank_cp<3, 64, 1> : k_gemm_bank_cp<2, 64, 1>;
     else if (shape == 3)
-        kern = S == 5 ? k_gemm_bank_cp<5, 64, 1, 16> : S == 4 ? k_gemm_bank_cp<4, 64, 1, 16>
-             : S == 3 ? k_gemm_bank_cp<3, 64, 1, 16> : k_gemm_bank_cp<2, 64, 1, 16>;
+        kern = S == 5 ? k_gemm_bank_cp<5, 64, 1, 8, 16> : S == 4 ? k_gemm_bank_cp<4, 64, 1, 8, 16>
+             : S == 3 ? k_gemm_bank_cp<3, 64, 1, 8, 16> : k_gemm_bank_cp<2, 64, 1, 8, 16>;
     else if (shape == 1) {
         S = S >= 9 ? 9 : S >= 8 ? 8 : S >= 6 ? 6 : S >= 4 ? 4 : 2;   // the instantiated depths
         kern = S == 9 ? k_gemm_bank_cp<9, 32, 1> : S == 8 ? k_gemm_bank_cp<8, 32, 1>
@@ -793,7 +850,7 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smemCp);
     if (e != cudaSuccess) return e;
-    kern<<<grid, cp_threads(shape == 3 ? 16 : 8), smemCp, st>>>(rowsOf, cBh, cBl, p);
+    kern<<<grid, cp_threads(8, shape == 3 ? 16 : 0), smemCp, st>>>(rowsOf, cBh, cBl, p);
     return cudaGetLastError();
 }
 

@@ -495,12 +495,12 @@ bool bf16x3_available();
 // rows' norms sum_p sigRcp ctf^2 |P|^2 (compensated FP32).  shape (the
 // cp.async form): 0 K blocks of 64 bf16, one CTA an SM; 1 K blocks of 32,
 // twice the stages; 2 K blocks of 32, two CTAs an SM; 3 as 0 with 16
-// gather warps instead of 8.
+// norm warps beside the 8 that gather.  wn: scratch of nP Kd / 2 floats.
 cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const int* idx,
                                     const int* cls, int nP, int nR, const void* B, int nT,
                                     int Kd, int K, const float* sigRcp, const float* ctf,
                                     float* C, float alpha, int* flag, cudaStream_t st,
-                                    bool tmaGather = false, int* order = nullptr, int shape = 3);
+                                    bool tmaGather, int* order, int shape, float* wn);
 cudaError_t launch_gemm_nt_bf16x3(const float* A, long long sA, int lda,
                                   const float* B, long long sB, int ldb,
                                   int M, int N, int Kd, int batch, float* C,
