@@ -169,11 +169,37 @@ static int check_weights_shape(int nR, int nT)
     return TG3_OK;
 }
 
+// Pinned host memory of a context for a call's inputs (packed, one copy) and
+// outputs: bytes after the head.  A call that used it ends with its stream
+// synchronised.
+constexpr size_t kPinHead = 64, kPinFirst = 256 * 1024;
+
+static char* pin_get(tg3_ctx* c, size_t bytes, int* status)
+{
+    if (c->pinBytes < bytes + kPinHead) {
+        cudaError_t e = cudaStreamSynchronize(c->stream);
+        cudaFreeHost(c->pin);
+        c->pin = nullptr;
+        c->pinBytes = 0;
+        if (e == cudaSuccess) e = cudaMallocHost((void**)&c->pin, bytes + kPinHead);
+        if (e != cudaSuccess) {
+            c->pin = nullptr;
+            *status = cuda_fail(e, "cudaMallocHost");
+            return nullptr;
+        }
+        c->pinBytes = bytes + kPinHead;
+    }
+    return c->pin + kPinHead;
+}
+
 static int sync_and_check(tg3_ctx* c)
 {
+    int st = TG3_OK;
+    if (!pin_get(c, 0, &st)) return st;
+    int* word = reinterpret_cast<int*>(c->pin);
+    TG3_CUDA(cudaMemcpyAsync(word, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     TG3_CUDA(cudaStreamSynchronize(c->stream));
-    int flag = 0;
-    TG3_CUDA(cudaMemcpy(&flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
+    const int flag = *word;
     if (flag) {
         TG3_CUDA(cudaMemset(c->d_flag, 0, sizeof(int)));
         if (flag & 1) return fail(TG3_ERR_ARG, "resampling permutation out of range");
@@ -285,6 +311,10 @@ extern "C" int tg3_ctx_create(tg3_ctx** out, int device)
     if (e == cudaSuccess) e = cudaMalloc(&c->d_volTable, sizeof(float4*) * kMaxClasses);
     if (e == cudaSuccess) e = cudaMemset(c->d_volTable, 0, sizeof(float4*) * kMaxClasses);
     if (e == cudaSuccess) e = prefer_carveouts();
+    if (e == cudaSuccess) {
+        e = cudaMallocHost((void**)&c->pin, kPinFirst);   // enough for a particle's usual call
+        if (e == cudaSuccess) c->pinBytes = kPinFirst;
+    }
     if (e != cudaSuccess) {
         int st = cuda_fail(e, "context set-up");
         tg3_ctx_destroy(c);
@@ -313,6 +343,7 @@ extern "C" int tg3_ctx_destroy(tg3_ctx* c)
     }
     cudaFree(c->ins.acc);
     cudaFree(c->ins.tab);
+    cudaFreeHost(c->pin);
     for (auto& b : c->bank) {
         cudaFree(b.f32);
         cudaFree(b.hi);
@@ -1448,32 +1479,37 @@ extern "C" int tg3_ExpectLocal3D(tg3_volume* h, const float* dat, const float* c
            owt = ar.add(8 * (size_t)nT), obl = ar.add(8), odv = ar.add(4 * (size_t)nR * nT);
     char* b = (char*)ws_get(c, WS_H2D, ar.used, &st);
     if (!b) return st;
-    TG3_CUDA(cudaMemcpyAsync(b + od, dat, 8 * (size_t)K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + oc, ctf, 4 * (size_t)K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + os, sigRcp, 4 * (size_t)K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + oq, rot, 32 * (size_t)nR, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + ot, trans, 16 * (size_t)nT, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opr, oldR, 8 * (size_t)nR, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opt, oldT, 8 * (size_t)nT, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opc, &oldC, 8, cudaMemcpyHostToDevice, s));
+    // the inputs go over in one copy and the results come back in one: thirteen
+    // small copies were most of the call
+    char* pin = pin_get(c, odv, &st);
+    if (!pin) return st;
+    std::memcpy(pin + od, dat, 8 * (size_t)K);
+    std::memcpy(pin + oc, ctf, 4 * (size_t)K);
+    std::memcpy(pin + os, sigRcp, 4 * (size_t)K);
+    std::memcpy(pin + oq, rot, 32 * (size_t)nR);
+    std::memcpy(pin + ot, trans, 16 * (size_t)nT);
+    std::memcpy(pin + opr, oldR, 8 * (size_t)nR);
+    std::memcpy(pin + opt, oldT, 8 * (size_t)nT);
+    std::memcpy(pin + opc, &oldC, 8);
+    TG3_CUDA(cudaMemcpyAsync(b, pin, owc, cudaMemcpyHostToDevice, s));
     st = local_phase(c, nullptr, 1, nR, nT, (float*)(b + od), (float*)(b + oc), (float*)(b + os),
                      (double*)(b + oq), (double*)(b + ot), (double*)(b + opr), (double*)(b + opt),
                      (double*)(b + opc), nullptr, (double*)(b + owc), (double*)(b + owr),
                      (double*)(b + owt), (double*)(b + obl), dvp ? (float*)(b + odv) : nullptr,
                      TG3_SCORE_FP32);
-    if (st) return st;
-    std::vector<double> hwr(nR), hwt(nT);
-    double hwc = 0, hbl = 0;
-    TG3_CUDA(cudaMemcpyAsync(hwr.data(), b + owr, 8 * (size_t)nR, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(hwt.data(), b + owt, 8 * (size_t)nT, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(&hwc, b + owc, 8, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(&hbl, b + obl, 8, cudaMemcpyDeviceToHost, s));
+    if (st) {
+        cudaStreamSynchronize(s);      // the copy out of pin
+        return st;
+    }
+    TG3_CUDA(cudaMemcpyAsync(pin + owc, b + owc, odv - owc, cudaMemcpyDeviceToHost, s));
     if (dvp) TG3_CUDA(cudaMemcpyAsync(dvp, b + odv, 4 * (size_t)nR * nT, cudaMemcpyDeviceToHost, s));
     if ((st = sync_and_check(c))) return st;
+    const double* hwr = reinterpret_cast<const double*>(pin + owr);
+    const double* hwt = reinterpret_cast<const double*>(pin + owt);
     for (int r = 0; r < nR; r++) wR[r] = (float)hwr[r];
     for (int t = 0; t < nT; t++) wT[t] = (float)hwt[t];
-    *wC = (float)hwc;
-    *baseL = (float)hbl;
+    *wC = (float)*reinterpret_cast<const double*>(pin + owc);
+    *baseL = (float)*reinterpret_cast<const double*>(pin + obl);
     return TG3_OK;
 }
 
@@ -1505,23 +1541,27 @@ extern "C" int tg3_ExpectLocal3D_ctf(tg3_volume* h, const float* dat, const floa
     const size_t K = npxl, R_ = nR, T_ = nT, D_ = nD;
     Arena ar(c, WS_H2D);
     size_t od = ar.add(8 * K), odo = ar.add(4 * K), ofq = ar.add(4 * K), os = ar.add(4 * K),
-           octf = ar.add(4 * K * D_), oq = ar.add(32 * R_), ot = ar.add(16 * T_),
+           oq = ar.add(32 * R_), ot = ar.add(16 * T_),
            odp = ar.add(8 * D_), opr = ar.add(8 * R_), opt = ar.add(8 * T_), opd = ar.add(8 * D_),
            opc = ar.add(8), owc = ar.add(8), owr = ar.add(8 * R_), owt = ar.add(8 * T_),
-           owd = ar.add(8 * D_), obl = ar.add(8), odv = ar.add(dvp ? 4 * D_ * R_ * T_ : 0);
+           owd = ar.add(8 * D_), obl = ar.add(8), octf = ar.add(4 * K * D_),
+           odv = ar.add(dvp ? 4 * D_ * R_ * T_ : 0);
     char* b = (char*)ws_get(c, WS_H2D, ar.used, &st);
     if (!b) return st;
-    TG3_CUDA(cudaMemcpyAsync(b + od, dat, 8 * K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + odo, defO, 4 * K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + ofq, freQ, 4 * K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + os, sigRcp, 4 * K, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + oq, rot, 32 * R_, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + ot, trans, 16 * T_, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + odp, dpara, 8 * D_, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opr, oldR, 8 * R_, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opt, oldT, 8 * T_, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opd, oldD, 8 * D_, cudaMemcpyHostToDevice, s));
-    TG3_CUDA(cudaMemcpyAsync(b + opc, &oldC, 8, cudaMemcpyHostToDevice, s));
+    char* pin = pin_get(c, octf, &st);
+    if (!pin) return st;
+    std::memcpy(pin + od, dat, 8 * K);
+    std::memcpy(pin + odo, defO, 4 * K);
+    std::memcpy(pin + ofq, freQ, 4 * K);
+    std::memcpy(pin + os, sigRcp, 4 * K);
+    std::memcpy(pin + oq, rot, 32 * R_);
+    std::memcpy(pin + ot, trans, 16 * T_);
+    std::memcpy(pin + odp, dpara, 8 * D_);
+    std::memcpy(pin + opr, oldR, 8 * R_);
+    std::memcpy(pin + opt, oldT, 8 * T_);
+    std::memcpy(pin + opd, oldD, 8 * D_);
+    std::memcpy(pin + opc, &oldC, 8);
+    TG3_CUDA(cudaMemcpyAsync(b, pin, owc, cudaMemcpyHostToDevice, s));
     TG3_CUDA(launch_ctf_defocus((float*)(b + odo), (float*)(b + ofq), (double*)(b + odp), nD,
                                 npxl, k1, k2, phaseShift, conT, (float*)(b + octf), s));
     st = local_phase_ctf(c, 1, nR, nT, nD, (float*)(b + od), (float*)(b + octf), (float*)(b + os),
@@ -1530,21 +1570,21 @@ extern "C" int tg3_ExpectLocal3D_ctf(tg3_volume* h, const float* dat, const floa
                          (double*)(b + owc), (double*)(b + owr), (double*)(b + owt),
                          (double*)(b + owd), (double*)(b + obl), dvp ? (float*)(b + odv) : nullptr,
                          TG3_SCORE_FP32);
-    if (st) return st;
-    std::vector<double> hwr(R_), hwt(T_), hwd(D_);
-    double hwc = 0, hbl = 0;
-    TG3_CUDA(cudaMemcpyAsync(hwr.data(), b + owr, 8 * R_, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(hwt.data(), b + owt, 8 * T_, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(hwd.data(), b + owd, 8 * D_, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(&hwc, b + owc, 8, cudaMemcpyDeviceToHost, s));
-    TG3_CUDA(cudaMemcpyAsync(&hbl, b + obl, 8, cudaMemcpyDeviceToHost, s));
+    if (st) {
+        cudaStreamSynchronize(s);      // the copy out of pin
+        return st;
+    }
+    TG3_CUDA(cudaMemcpyAsync(pin + owc, b + owc, octf - owc, cudaMemcpyDeviceToHost, s));
     if (dvp) TG3_CUDA(cudaMemcpyAsync(dvp, b + odv, 4 * D_ * R_ * T_, cudaMemcpyDeviceToHost, s));
     if ((st = sync_and_check(c))) return st;
+    const double* hwr = reinterpret_cast<const double*>(pin + owr);
+    const double* hwt = reinterpret_cast<const double*>(pin + owt);
+    const double* hwd = reinterpret_cast<const double*>(pin + owd);
     for (int r = 0; r < nR; r++) wR[r] = (float)hwr[r];
     for (int t = 0; t < nT; t++) wT[t] = (float)hwt[t];
     for (int d = 0; d < nD; d++) wD[d] = (float)hwd[d];
-    *wC = (float)hwc;
-    *baseL = (float)hbl;
+    *wC = (float)*reinterpret_cast<const double*>(pin + owc);
+    *baseL = (float)*reinterpret_cast<const double*>(pin + obl);
     return TG3_OK;
 }
 

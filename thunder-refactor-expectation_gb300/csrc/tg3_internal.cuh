@@ -201,6 +201,8 @@ struct tg3_ctx {
     unsigned pixGen = 0;                     // pixel uploads so far
     tg3::Buffer ws[tg3::WS_COUNT];
     int* d_flag = nullptr;           // device error word
+    char* pin = nullptr;             // pinned staging of the host-array calls (grow-only), its
+    size_t pinBytes = 0;             // first kPinHead bytes for the error word
     // tg3_ctx_set_option
     bool fused = false;
     bool insertGather = false;    // TG3_OPT_INSERT_GATHER
