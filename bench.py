@@ -1119,7 +1119,7 @@ def run_reco(args, rank, world, local_rank):
             "config": {"workload": "reco256", "box": N, "pf": pf, "max_radius": maxR,
                        "balancing_rounds": rounds, "l2": "arrays (2.7 GB) larger than L2"},
             "clocks": clocks,
-            "roofline": {"bound": "hbm", "kernel": "whole reconstruction (cuFFT-dominated)",
+            "roofline": {"bound": "hbm", "kernel": "whole reconstruction",
                          "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                          "frac": round(achieved / hbm, 4), "peak_kind": kind, "traffic": None}}
 
