@@ -2050,7 +2050,7 @@ k_resample(int ld, const double* __restrict__ uIn, const double* __restrict__ wI
 // before one atomic per component, and the draw counter.
 // With nC (the multi-class InsertFT), draw m of image l is inserted only
 // when m < nC[l] (kernel_getRandomR / kernel_InsertF, gpu/src/Kernel.cu:
-// 1847-1899, 2552-2600): a skipped draw gets weight 0, which k_insert
+// 1847-1899, 2552-2600): a skipped draw gets weight 0, which the insertion
 // skips, and adds nothing to O3D or the counter.
 __global__ void __launch_bounds__(256)
 k_insert_draws(int nDraws, int drawsPerImage, const double* __restrict__ quat,

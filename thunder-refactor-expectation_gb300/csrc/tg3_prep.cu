@@ -892,7 +892,11 @@ extern "C" int tg3_prepare_images_d(tg3_ctx* c, const float* img, int nImg, int 
     const PrepTables tabs{(float*)(b + oM), sm.qIn, nMask, r, ew, (float2*)(b + oT), pl.A, pl.B,
                           (int*)(b + oL), c->px.iCol, c->px.iRow, pl.A ? K : 0, pl.cols, maxCol,
                           pl.W};
-    k_bg_stats<<<nImg, 256, sizeof(int2) * up(N), s>>>(img, N, bgAbove, (double)cnt, stv, stats, tabs);
+    const size_t rowsB = sizeof(int2) * ((size_t)(N + 3) / 4 * 4);
+    if (rowsB > 47 * 1024)
+        TG3_CUDA(cudaFuncSetAttribute(k_bg_stats, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)rowsB));
+    k_bg_stats<<<nImg, 256, rowsB, s>>>(img, N, bgAbove, (double)cnt, stv, stats, tabs);
     TG3_LAUNCH_CHECK("background statistics");
     k_stdn<<<1, 256, 0, s>>>(stv, nImg, stdN, sc);
     TG3_LAUNCH_CHECK("noise level");
