@@ -769,9 +769,7 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
         while (n2 < nP) n2 <<= 1;
         const size_t sm = sizeof(unsigned long long) * n2;
         if (sm > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(k_bank_order,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)sm);
+            cudaError_t e = allow_shared(k_bank_order);
             if (e != cudaSuccess) return e;
         }
         k_bank_order<<<1, 1024, sm, st>>>(idx, cls, nP, nR, n2, order);
@@ -796,9 +794,7 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
     const size_t smem = 1024 + (size_t)p.stages * stageBytes + 256 + 2 * sizeof(int) * BG_M;
     dim3 grid((nR + BG_M - 1) / BG_M, nP);
     if (tmaGather) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_bank_bf16x3,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        cudaError_t e = allow_shared(k_gemm_bank_bf16x3);
         if (e != cudaSuccess) return e;
         k_gemm_bank_bf16x3<<<grid, BG_THREADS, smem, st>>>(maps, mBh, mBl, p);
         return cudaGetLastError();
@@ -847,8 +843,7 @@ cudaError_t launch_gemm_bank_bf16x3(const Bank* banks, unsigned pixGen, const in
                      !tc::make_map(&cBl, Bl, (long long)nP * nT, Kd, p.ntile, 32, true)))
         return cudaErrorInvalidValue;
     const size_t smemCp = fixed + (size_t)S * stageCp;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smemCp);
+    cudaError_t e = allow_shared(kern);
     if (e != cudaSuccess) return e;
     kern<<<grid, cp_threads(8, shape == 3 ? 16 : 0), smemCp, st>>>(rowsOf, cBh, cBl, p);
     return cudaGetLastError();

@@ -1165,8 +1165,7 @@ extern "C" int tg3_cnn_match_propose(const float* out, int n, const float* ref, 
     while (p2 < nRot) p2 <<= 1;
     const size_t smem = sizeof(unsigned long long) * p2 + sizeof(uint32_t) * (size_t)nRef;
     if (smem > 200 * 1024) return fail(TG3_ERR_ARG, "match sizes need too much shared memory");
-    TG3_CUDA(cudaFuncSetAttribute(k_match_propose, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
+    TG3_CUDA(allow_shared(k_match_propose));
     k_match_propose<<<n, 256, smem, static_cast<cudaStream_t>(stream)>>>(
         out, ref, nRef, p2, refQuat, nRot, nTrans, seed, quat, trans, idx, nullptr, nullptr);
     TG3_LAUNCH_CHECK("match proposals");
@@ -1186,8 +1185,7 @@ cudaError_t tg3::launch_match_propose_classes(const float* out, int n, const Ref
     while (p2 < nRot) p2 <<= 1;
     const size_t smem = sizeof(unsigned long long) * p2 + sizeof(uint32_t) * (size_t)maxRef;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_match_propose,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(k_match_propose);
     if (e != cudaSuccess) return e;
     k_match_propose<<<n, 256, smem, st>>>(out, nullptr, maxRef, p2, nullptr, nRot, nTrans, seed,
                                           quat, trans, idx, table, cls);

@@ -329,8 +329,7 @@ cudaError_t launch_conv_tc(const ConvTcArgs& a, cudaStream_t st)
         a.coutPad < 16 || a.coutPad > 256 || a.tmemCols < a.coutPad)
         return cudaErrorInvalidValue;
     const size_t smem = conv_tc_smem(a.coutPad);
-    cudaError_t e = cudaFuncSetAttribute(k_conv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_shared(k_conv_tc);
     if (e != cudaSuccess) return e;
     if (a.kSplit < 1 || a.kSplit > 65535 || (a.kSplit > 1 && !a.partial))
         return cudaErrorInvalidValue;

@@ -454,7 +454,7 @@ size_t fused_smem_bytes(int vdim, int ntile, int* stagesOut)
     const size_t tail = sizeof(int) * ((size_t)vdim / 2 + 1 + 2 * (size_t)vdim) +
                         sizeof(float) * (FU_M * 9 + FU_M + FU_ROWS * FU_WARPS * 16) + 8 +
                         16 * sizeof(uint64_t) + 12 * sizeof(int) + 16 + sizeof(ItemDesc);
-    const size_t limit = 227 * 1024;
+    const size_t limit = kSmemCta;
     for (int S = 3; S >= 2; S--) {
         const size_t total = 1024 + S * stageBytes + tail;
         if (total <= limit) {
@@ -512,8 +512,7 @@ cudaError_t launch_fused_bf16x3(float4* const* volTable, int vdim, int pf, const
     if (!tc::make_map(&mBh, Bh, rowsB, KpB, p.ntile, FU_BK, true) ||
         !tc::make_map(&mBl, Bl, rowsB, KpB, p.ntile, FU_BK, true))
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_fused_bf16x3,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(k_fused_bf16x3);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -41,6 +41,24 @@ int cuda_fail(cudaError_t e, const char* what);
         if (e_ != cudaSuccess) return ::tg3::cuda_fail(e_, what);        \
     } while (0)
 
+// Shared memory of a CTA (dynamic and static together) and of an SM.
+constexpr size_t kSmemCta = 227 * 1024, kSmemSm = 228 * 1024;
+
+// Lets kern be launched with all the dynamic shared memory that its static part
+// leaves.  The limit belongs to the function, not to a context or a stream:
+// a limit of this call's own size would be lowered under it by another
+// thread's smaller call, between here and the launch or the next round's.
+template <typename Kernel>
+inline cudaError_t allow_shared(Kernel kern)
+{
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kSmemCta - a.sharedSizeBytes));
+    return e;
+}
+
 // A float as an int in the same order (its own inverse on the way back); NaN
 // aside, the largest of floats is the largest of keys.
 __host__ __device__ __forceinline__ int float_key_bits(int b) { return b ^ ((b >> 31) & 0x7fffffff); }

@@ -2695,7 +2695,7 @@ cudaError_t launch_project(float4* const* volTable, const int* cls, const float4
                 : form == 1 ? k_project_lane<false>
                             : k_project;
     if (tabBytes > 48 * 1024) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tabBytes);
+        e = allow_shared(kern);
         if (e != cudaSuccess) return e;
     }
     kern<<<(unsigned)grid, 256, form == 4 ? 0 : tabBytes, st>>>(volTable, cls, vol, vdim, pf, mf, rowsPerParticle,
@@ -3054,8 +3054,7 @@ cudaError_t launch_resample(int nP, int n, const double* u, const double* w, con
 {
     size_t smem = sizeof(double) * (2 * (size_t)n + (size_t)(n > nOut ? n : nOut))
                 + sizeof(int) * (size_t)n;
-    cudaError_t e = cudaFuncSetAttribute(k_resample, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_shared(k_resample);
     if (e != cudaSuccess) return e;
     k_resample<<<nP, 256, smem, st>>>(n, u, w, perm, u0, peak, nOut, nPer, src, wOut, top, flag);
     return cudaGetLastError();
@@ -3086,8 +3085,7 @@ cudaError_t launch_insert(float4* acc, int vdim, int kernel, const float* tab, i
         const bool shared = smem <= 200 * 1024;
         const auto kern = shared ? k_insert_mkb<true> : k_insert_mkb<false>;
         if (shared) {
-            const cudaError_t e =
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            const cudaError_t e = allow_shared(kern);
             if (e != cudaSuccess) return e;
         }
         const long long items = (long long)((K + kInsertItem - 1) / kInsertItem) * nDraws;
@@ -3176,8 +3174,7 @@ cudaError_t launch_bank_gather(const BankView* table, const int* cls, const int*
     const size_t smem = sizeof(float) * (size_t)K;
     if (smem > 48 * 1024) {
         if (smem > 200 * 1024) return cudaErrorInvalidValue;
-        cudaError_t e = cudaFuncSetAttribute(k_bank_gather,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_shared(k_bank_gather);
         if (e != cudaSuccess) return e;
     }
     dim3 grid(nP, (nR + kBankRows - 1) / kBankRows);
@@ -3192,7 +3189,7 @@ cudaError_t launch_fsc(const float2* A, const float2* B, int vdim, int nShell, d
     cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(double) * 3 * (size_t)nShell, st);
     if (e != cudaSuccess) return e;
     const size_t smem = sizeof(double) * 3 * (size_t)nShell;
-    e = cudaFuncSetAttribute(k_fsc_shells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_shared(k_fsc_shells);
     if (e != cudaSuccess) return e;
     const size_t n = (size_t)vdim * vdim * (vdim / 2 + 1);
     k_fsc_shells<<<grid_for(n, 256, 152 * 4), 256, smem, st>>>(A, B, vdim, nShell, sums);

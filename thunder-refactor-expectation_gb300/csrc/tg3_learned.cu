@@ -376,8 +376,7 @@ static int learned_expect(tg3_ctx* c, tg3_cnn* net, int nP, const float* images,
         int p2 = 1;
         while (p2 < n) p2 <<= 1;
         const size_t smem = sizeof(float) * p2;
-        TG3_CUDA(cudaFuncSetAttribute(k_peak_score, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+        TG3_CUDA(allow_shared(k_peak_score));
         k_peak_score<<<nP, 512, smem, s>>>(dvp, n, p2, peak);
         TG3_LAUNCH_CHECK("proposal confidence");
         k_best_proposal<<<(nP + 7) / 8, 256, 0, s>>>(wR, wT, nP, nRot, nTrans, quat, trans, base,

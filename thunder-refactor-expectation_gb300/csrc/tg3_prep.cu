@@ -30,8 +30,6 @@
 namespace tg3 {
 namespace {
 
-constexpr size_t kSmemCta = 227 * 1024, kSmemSm = 228 * 1024;   // dynamic of a CTA; of an SM
-
 __device__ double prep_block_sum(double v, double* scratch)
 {
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -894,15 +892,13 @@ extern "C" int tg3_prepare_images_d(tg3_ctx* c, const float* img, int nImg, int 
                           pl.W};
     const size_t rowsB = sizeof(int2) * ((size_t)(N + 3) / 4 * 4);
     if (rowsB > 47 * 1024)
-        TG3_CUDA(cudaFuncSetAttribute(k_bg_stats, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)rowsB));
+        TG3_CUDA(allow_shared(k_bg_stats));
     k_bg_stats<<<nImg, 256, rowsB, s>>>(img, N, bgAbove, (double)cnt, stv, stats, tabs);
     TG3_LAUNCH_CHECK("background statistics");
     k_stdn<<<1, 256, 0, s>>>(stv, nImg, stdN, sc);
     TG3_LAUNCH_CHECK("noise level");
     if (pl.A)
-        TG3_CUDA(cudaFuncSetAttribute(k_prep_ft, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kSmemCta));
+        TG3_CUDA(allow_shared(k_prep_ft));
     for (int l0 = 0; l0 < nImg; l0 += IB) {
         const int n = std::min(IB, nImg - l0);
         float2* out = reinterpret_cast<float2*>(dat) + (size_t)l0 * K;

@@ -836,9 +836,9 @@ int reconstruct_passes(tg3_ctx* c, const PassKernels& k, const float4* acc, int 
     cudaStream_t s = c->stream;
     const size_t smemZ = k.smem + 2 * sizeof(float) * (size_t)n * kFftLines;
     const size_t smemX = k.smem + sizeof(float2) * 2 * kFftLines * ((p.px + 15) / 16 * 16 + 2);
-    TG3_CUDA(cudaFuncSetAttribute(k.y, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
-    TG3_CUDA(cudaFuncSetAttribute(k.x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemX));
-    TG3_CUDA(cudaFuncSetAttribute(k.z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemZ));
+    TG3_CUDA(allow_shared(k.y));
+    TG3_CUDA(allow_shared(k.x));
+    TG3_CUDA(allow_shared(k.z));
     const double i0a = bessel_i0(alpha), cellsD = (double)n * n * n;
     const double invNf = gridCorr ? 1.0 / mkb_rl(0.0, a, alpha, i0a) : 0.0;
     fft::k_roots<<<(n + 127) / 128, 128, 0, s>>>(const_cast<float2*>(p.tw), n);

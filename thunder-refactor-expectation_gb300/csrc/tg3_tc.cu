@@ -650,8 +650,7 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
             return cudaErrorInvalidValue;
         void (*kern)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                      const TcParams) = bk == 64 ? k_gemm_bf16x3_pair<64> : k_gemm_bf16x3_pair<32>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        cudaError_t e = allow_shared(kern);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)((mTiles + 1) / 2 * 2), (unsigned)items);
@@ -670,8 +669,7 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
     const size_t smem = (size_t)p.stages * stageBytes + extra;
     void (*kern)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                  const TcParams) = bk == 64 ? k_gemm_bf16x3<64> : k_gemm_bf16x3<32>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_shared(kern);
     if (e != cudaSuccess) return e;
     kern<<<std::min(p.tiles, 152), TC_THREADS, smem, st>>>(mAh, mAl, mBh, mBl, p);
     return cudaGetLastError();
