@@ -2375,8 +2375,7 @@ def main():
                     help="rescoring form (TG3_OPT_BANK_GATHER): 0 cross term gathers the bank "
                          "rows with cp.async, 1 rows copied out first, 2 TMA gathers")
     ap.add_argument("--scan-pair", type=int, default=0, choices=[0, 1],
-                    help="TG3_OPT_SCAN_PAIR: the global search's cross term on CTA pairs that "
-                         "share each column tile by TMA multicast")
+                    help="TG3_OPT_SCAN_PAIR: accepted, without effect")
     ap.add_argument("--local-bk", type=int, default=64, choices=[32, 64],
                     help="TG3_OPT_LOCAL_BK: K block of the local phase's split cross term")
     ap.add_argument("--bank-shape", type=int, default=3, choices=[0, 1, 2, 3],

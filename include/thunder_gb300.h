@@ -339,10 +339,8 @@ int tg3_ctx_set_timing(tg3_ctx* ctx, int enable);
  *   of 16 up to 256) of the split-bf16 global scan's cross term; a narrower
  *   tile leaves room for more pipeline stages.  The results do not depend on
  *   it.
- * TG3_OPT_SCAN_PAIR (default 0): 1 runs that cross term on pairs of CTAs
- *   (a thread-block cluster of two on neighbouring row tiles) that share
- *   each column tile: each CTA loads half of it, multicast to both, halving
- *   the bytes the column operand takes from L2.  Same results.
+ * TG3_OPT_SCAN_PAIR: accepted for programs that set it; either value runs
+ *   that cross term in its one form, a CTA per column tile.
  * TG3_OPT_SCAN_BK (default 32): the K block of that cross term's pipeline
  *   stages, 64 bf16 (128-byte rows, 128-byte swizzle) or 32 (64-byte rows,
  *   64-byte swizzle: half the bytes a stage, twice the stages in flight).

@@ -1849,7 +1849,7 @@ extern "C" int tg3_ctx_set_option(tg3_ctx* c, int option, int value)
             return fail(TG3_ERR_ARG, "TG3_OPT_SCAN_TILE_N takes 0 or a multiple of 16 up to 256");
         c->scanTileN = value;
     }
-    else if (option == TG3_OPT_SCAN_PAIR) c->scanPair = value != 0;
+    else if (option == TG3_OPT_SCAN_PAIR) {}   // no form of its own
     else if (option == TG3_OPT_SCAN_BK) {
         if (value != 32 && value != 64) return fail(TG3_ERR_ARG, "TG3_OPT_SCAN_BK takes 32 or 64");
         c->scanBK = value;
@@ -2066,7 +2066,7 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                                        &st);
     if (!img2 && !pbank && !pscr) return st;
     int* best = nullptr;
-    if (split && !c->scanPair) {
+    if (split) {
         best = (int*)ws_get(c, WS_BEST, sizeof(int) * (size_t)IB * std::max(nK, 16), &st);
         if (!best) return st;
     }
@@ -2144,7 +2144,7 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                 const int Nn = std::min(256, (n + 15) / 16 * 16);
                 const int itemsN = (n + Nn - 1) / Nn;
                 TG3_CUDA(launch_gemm_bf16x3(abs2, nRt, sc2, n, nRt, Nn, Kq, itemsN, 0, Nn, n, nrmG,
-                                            Nn, n, nullptr, 0, 1.0f, c->d_flag, s, 0, 0, false,
+                                            Nn, n, nullptr, 0, 1.0f, c->d_flag, s, 0, 0,
                                             Kq % c->scanBK == 0 ? c->scanBK : 64));
             } else if ((st = norm_gemm(c, abs2, sc2, nRt, n, Kq, nrmG, s))) {
                 return st;
@@ -2163,8 +2163,7 @@ static int global_scan(tg3_ctx* c, const Volume* v, const float2* img2, int vdim
                 const int items = (cols + Nt - 1) / Nt;
                 TG3_CUDA(launch_gemm_bf16x3(P, nRt, A, (long long)cols, nRt, Nt, Kp, items, 0, Nt,
                                             cols, D, 0, nT, nullptr, 0, -2.0f, c->d_flag, s, nT,
-                                            (long long)nRt * nT, c->scanPair != 0,
-                                            Kp % c->scanBK == 0 ? c->scanBK : 64,
+                                            (long long)nRt * nT, Kp % c->scanBK == 0 ? c->scanBK : 64,
                                             best ? &tb : nullptr));
             } else {
                 TG3_CUDA(launch_gemm_nt_fp32(P, 0, Kp, A, 0, Kp, nRt, cols, Kp, 1, D, 0, nT,

@@ -227,7 +227,6 @@ struct tg3_ctx {
     int bankGather = 0;           // TG3_OPT_BANK_GATHER (0, 1 or 2)
     int bankOrder = 1;            // TG3_OPT_BANK_ORDER
     int scanTileN = 0;            // TG3_OPT_SCAN_TILE_N (0: 256)
-    int scanPair = 0;             // TG3_OPT_SCAN_PAIR
     int scanBK = 32;              // TG3_OPT_SCAN_BK
     int localBK = 64;             // TG3_OPT_LOCAL_BK
     int projForm = 4;             // TG3_OPT_PROJECT_FORM
@@ -552,8 +551,7 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
                                int bRowsPerItem, int nTotal, float* C, long long sC, int ldc,
                                const float* nrm, long long sN, float alpha, int* flag,
                                cudaStream_t st, int cGroup = 0, long long cGroupStride = 0,
-                               bool pair = false, int bk = 64, const TileBest* best = nullptr,
-                               bool besideProjections = false);
+                               int bk = 64, const TileBest* best = nullptr, bool besideProjections = false);
 // Shared-memory preferences of the kernels that run beside projections, for
 // the current device.
 cudaError_t prefer_carveouts();
