@@ -59,8 +59,9 @@ inline cudaError_t allow_shared(Kernel kern)
     return e;
 }
 
-// A float as an int in the same order (its own inverse on the way back); NaN
-// aside, the largest of floats is the largest of keys.
+// A float as an int in the same order (its own inverse on the way back): the
+// largest of floats is the largest of keys.  Not for NaN, whose keys lie past
+// the infinities': the caller skips it.
 __host__ __device__ __forceinline__ int float_key_bits(int b) { return b ^ ((b >> 31) & 0x7fffffff); }
 #ifdef __CUDACC__
 __device__ __forceinline__ int float_key(float x) { return float_key_bits(__float_as_int(x)); }

@@ -94,7 +94,8 @@ __device__ __forceinline__ void load_norms(const TcParams& p, float* ad, int lan
 // Largest value of each of the chunk's column groups (columns c0 .. c0 + cn - 1
 // of the tile, v[] of this lane's row) with the row's norm, then over the
 // warp's rows of every row group, into best.  fl(x + norm) grows with x, so the
-// norm is added to the largest x only.
+// norm is added to the largest x only.  A sum that is not a number is no maximum
+// (fmaxf over the columns skips one, and so does the weights' own pass).
 __device__ __forceinline__ void chunk_best(const TcParams& p, const float* v, int cn, const float* ad,
                                            int lane, int rowBase, int rows, int j0, int c0)
 {
@@ -107,7 +108,8 @@ __device__ __forceinline__ void chunk_best(const TcParams& p, const float* v, in
     auto put = [&](float m) {                                   // m: group l's largest of the row
         const float n = l - lTile < TC_SEGS ? ad[(l - lTile) * 32 + lane]
                                             : p.bestNrm[(size_t)min(row, p.M - 1) * p.bestNs + l];
-        const int key = float_key(m + n);
+        const float sum = m + n;
+        const int key = sum == sum ? float_key(sum) : kFloatKeyNegInf;
         for (int k = g0; k <= g1; k++) {
             const int top = __reduce_max_sync(0xffffffffu, g == k ? key : kFloatKeyNegInf);
             if (lane == 0) atomicMax(p.best + (size_t)l * p.bestGroups + k, top);
