@@ -703,6 +703,7 @@ struct tg3_cnn {
     float* wtrain = nullptr;
     size_t wFwd[kLayers] = {}, wBwd[kLayers] = {};
     bool wStale = true;
+    float* gradParts = nullptr; // the CTAs' parts of a convolution's weight gradient
     float* fcT = nullptr;       // wide dense layer's gradient: transposes, its sum
     int cap = 0;                // images the activation buffers hold
     float* act[kLayers + 1] = {};   // act[0] input copy .. act[8] outputs
@@ -827,6 +828,8 @@ int forward(tg3_cnn* net, int n)
 int backward(tg3_cnn* net, int n)
 {
     cudaStream_t s = net->stream;
+    if (!net->gradParts)
+        TG3_CUDA(cudaMalloc(&net->gradParts, sizeof(float) * conv_grad_part_floats()));
     for (int l = kLayers - 1; l >= 0; l--) {
         const LayerShape& sh = kShape[l];
         const float* W = net->params + net->off[l][0];
@@ -838,7 +841,8 @@ int backward(tg3_cnn* net, int n)
             k_relu_bwd<<<cnn_grid(cnt, 256), 256, 0, s>>>(gy, net->act[l + 1], cnt);
         }
         if (sh.stride) {
-            TG3_CUDA(launch_conv_bwd_weight(l, net->act[l], gy, dW, db, n, sh.cin, sh.cout, s));
+            TG3_CUDA(launch_conv_bwd_weight(l, net->act[l], gy, dW, db, n, sh.cin, sh.cout,
+                                            net->gradParts, s));
             if (l > 0)
                 TG3_CUDA(launch_conv_bwd_data(l, gy, net->wtrain + net->wBwd[l], net->act[l],
                                               net->gact[l], n, sh.cin, sh.cout, s));
@@ -945,6 +949,7 @@ extern "C" int tg3_cnn_destroy(tg3_cnn* net)
     cudaFree(net->loss);
     cudaFree(net->wtrain);
     cudaFree(net->fcT);
+    cudaFree(net->gradParts);
     cudaFree(net->emb);
     cudaFree(net->embLoss);
     cudaFree(net->tcW);

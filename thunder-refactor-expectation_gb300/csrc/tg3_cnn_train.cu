@@ -340,7 +340,36 @@ k_conv_classes(const ConvArgs p)
 // pixels a lane reads 32 gradients (uniform over the warp) and 18 (S 1) or 27
 // (S 2) inputs for 144 paired multiply-adds.  Chunks go through two shared
 // buffers by cp.async; the channel pitch over 4 is odd, so a quarter warp's
-// float4 reads fall in distinct banks.  One atomic add a sum and CTA.
+// float4 reads fall in distinct banks.
+//
+// Sums of a batch are long (262,144 terms a weight at 256 images of 32 x 32
+// pixels), so they are taken in three steps: a thread's FP32 chains end after
+// kGradChain terms and are added to its place in the CTA's part (global memory,
+// which stays in L2), and the CTAs' parts meet in FP64 in a fixed order
+// (k_grad_sum).  Error of a layer's gradient at 256 images, restated on the CPU:
+// 0.9 to 1.3e-7 of its norm; with one chain a CTA and atomic adds 2.0 to 3.8e-7.
+constexpr int kGradChain = 64;                               // a multiple of a chunk's 32
+constexpr int kGradPart = 72 * 128;                          // sums of a CTA
+constexpr int kGradCtas = 320;                               // most CTAs of a launch
+
+// the CTA's sums v[i][k] added to its part (or the first of it)
+__device__ __forceinline__ void add_to_part(uint64_t (&acc)[8][9], float* part, bool first)
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        float old[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) old[k] = first ? 0.f : part[(i * 9 + k) * 128];
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            const float2 v = unpack2(acc[i][k]);
+            const float s = v.x + v.y + old[k];
+            part[(i * 9 + k) * 128] = s;
+            acc[i][k] = 0ull;
+        }
+    }
+}
+
 template <int S, int HO>
 struct GradShape {
     static constexpr int RT = 64 / HO;                       // output rows of a chunk
@@ -356,8 +385,8 @@ struct GradShape {
 
 template <int S, int HO>
 __global__ void __launch_bounds__(128, 2)
-k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dW,
-            float* __restrict__ db, int n, int cin, int cout)
+k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ parts,
+            float* __restrict__ biasParts, int n, int cin, int cout)
 {
     using G = GradShape<S, HO>;
     constexpr int HI = G::HI, CPI = HO / G::RT;              // chunks of an image
@@ -394,8 +423,11 @@ k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __
     for (int i = 0; i < 8; i++)
 #pragma unroll
         for (int k = 0; k < 9; k++) acc[i][k] = 0ull;
-    float sb = 0.f;
+    double sb = 0.0;
     const bool bias = blockIdx.y == 0;
+    float* part = parts + ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x * kGradPart +
+                  (size_t)blockIdx.x * kGradPart + tid;
+    bool first = true;
     if (c0 < c1) stage(c0, 0);
     for (int ch = c0; ch < c1; ch++) {
         const int buf = (ch - c0) & 1;
@@ -408,6 +440,7 @@ k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __
         __syncthreads();
         const float* xb = xs + buf * G::XS + lane * G::CS;
         const float* yb = ys + buf * G::YS + warp * 8 * 64;
+        float sc = 0.f;
 #pragma unroll 1
         for (int q = 0; q < 16; q++) {
             const int oy = q / (HO / 4), c4 = 4 * (q % (HO / 4));
@@ -417,7 +450,7 @@ k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __
                 g[i] = *reinterpret_cast<const ulonglong2*>(yb + i * 64 + 4 * q);
             if (bias) {
                 const float4 t = *reinterpret_cast<const float4*>(yb + (lane & 7) * 64 + 4 * q);
-                sb += (t.x + t.y) + (t.z + t.w);
+                sc += (t.x + t.y) + (t.z + t.w);
             }
 #pragma unroll
             for (int r = 0; r < 3; r++) {
@@ -450,36 +483,39 @@ k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __
             }
         }
         __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            const float2 v = unpack2(acc[i][k]);
-            atomicAdd(dW + ((size_t)(co0 + warp * 8 + i) * cin + ci0 + lane) * 9 + k, v.x + v.y);
+        sb += sc;
+        if ((ch + 1 - c0) % (kGradChain / 32) == 0 || ch + 1 == c1) {
+            add_to_part(acc, part, first);
+            first = false;
         }
-    if (bias && lane < 8) atomicAdd(db + co0 + warp * 8 + lane, sb);
+    }
+    if (bias && lane < 8) biasParts[(size_t)blockIdx.z * cout + co0 + warp * 8 + lane] = (float)sb;
 }
 
 // The first layer's weight gradient (one input channel, 64 x 64): a lane per
 // 4 neighbouring pixels, straight from global memory (each gradient is read
-// once: bound by HBM); the warp's sums meet by shuffles at the end.
+// once: bound by HBM).  Chains and parts as above; a part has a sum of
+// every lane.
 __global__ void __launch_bounds__(128, 2)
-k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dW,
-             float* __restrict__ db, int n)
+k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ parts,
+             float* __restrict__ biasParts, int n)
 {
     constexpr int H = 64, GR = H * H / 4;                    // groups of 4 pixels an image
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t acc[8][9];
     float sb[8];
+    double sum[8] = {};
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         sb[i] = 0.f;
 #pragma unroll
         for (int k = 0; k < 9; k++) acc[i][k] = 0ull;
     }
-    const int total = n * GR;
-    for (int e = blockIdx.x * 32 + lane; e < total; e += gridDim.x * 32) {
+    float* part = parts + (size_t)blockIdx.x * kGradPart + threadIdx.x;
+    const int total = n * GR, step = gridDim.x * 32;
+    bool first = true;
+    int done = 0;
+    for (int e = blockIdx.x * 32 + lane; e < total; e += step) {
         const int im = e / GR, oy = e % GR / (H / 4), c4 = 4 * (e % (H / 4));
         const float* yp = dy + ((size_t)im * 32 + warp * 8) * (H * H) + oy * H + c4;
         ulonglong2 g[8];
@@ -507,20 +543,57 @@ k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* _
                     fma2(acc[i][3 * r + c], g[i].y, t[c][1]);
                 }
         }
+        if (++done % (kGradChain / 2) == 0 || e + step >= total) {
+            add_to_part(acc, part, first);
+            first = false;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                sum[i] += sb[i];
+                sb[i] = 0.f;
+            }
+        }
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            const float2 v = unpack2(acc[i][k]);
-            float s = v.x + v.y;
-            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) atomicAdd(dW + (size_t)(warp * 8 + i) * 9 + k, s);
-        }
-        float s = sb[i];
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) atomicAdd(db + warp * 8 + i, s);
+        for (int o = 16; o; o >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+        if (lane == 0) biasParts[(size_t)blockIdx.x * 32 + warp * 8 + i] = (float)sum[i];
     }
+}
+
+// dW += the sum of Z CTAs' parts [z][blocks][kGradPart] and db += that of
+// biasParts [z][cout], in FP64 and always in the same order.  CTA: 32 sums, 8
+// shares of the parts; the last cout / 32 CTAs have the biases.  With lanes
+// (the first layer) the 32 sums are the lanes' of one weight.
+__global__ void __launch_bounds__(256)
+k_grad_sum(const float* __restrict__ parts, const float* __restrict__ biasParts, int Z, int cin,
+           int cout, int lanes, float* __restrict__ dW, float* __restrict__ db)
+{
+    __shared__ double red[8][32];
+    const int t = threadIdx.x & 31, share = threadIdx.x >> 5;
+    const int xb = cout / 32, blocks = lanes ? 1 : xb * (cin / 32), nW = blocks * (kGradPart / 32);
+    const bool bias = (int)blockIdx.x >= nW;
+    const int e = ((int)blockIdx.x - (bias ? nW : 0)) * 32 + t;
+    const size_t pitch = bias ? (size_t)cout : (size_t)blocks * kGradPart;
+    const float* src = (bias ? biasParts : parts) + e;
+    double s = 0.0;
+#pragma unroll 8
+    for (int z = share; z < Z; z += 8) s += __ldg(src + z * pitch);
+    red[share][t] = s;
+    __syncthreads();
+    if (share) return;
+    for (int i = 1; i < 8; i++) s += red[i][t];
+    if (bias) {
+        db[e] += (float)s;
+        return;
+    }
+    const int b = e / kGradPart, j = e % kGradPart;
+    const int ik = j / 128, co = b % xb * 32 + j % 128 / 32 * 8 + ik / 9, ci = b / xb * 32 + t;
+    if (!lanes) {
+        dW[((size_t)co * cin + ci) * 9 + ik % 9] += (float)s;
+        return;
+    }
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (t == 0) dW[co * 9 + ik % 9] += (float)s;
 }
 
 // ------------------------------------------------------------ weight layout --
@@ -596,9 +669,17 @@ cudaError_t run_classes(const ConvArgs& a, cudaStream_t st)
     return cudaGetLastError();
 }
 
+cudaError_t sum_grad(const float* parts, const float* biasParts, int Z, int cin, int cout, int lanes,
+                     float* dW, float* db, cudaStream_t st)
+{
+    const int sums = (lanes ? 1 : (cout / 32) * (cin / 32)) * kGradPart + cout;
+    k_grad_sum<<<sums / 32, 256, 0, st>>>(parts, biasParts, Z, cin, cout, lanes, dW, db);
+    return cudaGetLastError();
+}
+
 template <int S, int HO>
 cudaError_t run_grad(const float* x, const float* dy, float* dW, float* db, int n, int cin,
-                     int cout, cudaStream_t st)
+                     int cout, float* parts, cudaStream_t st)
 {
     using G = GradShape<S, HO>;
     cudaError_t e = set_smem(k_conv_grad<S, HO>, G::bytes);
@@ -606,9 +687,12 @@ cudaError_t run_grad(const float* x, const float* dy, float* dW, float* db, int 
     // two CTAs an SM share the chunks
     const int blocks = (cout / 32) * (cin / 32), chunks = n * (HO / G::RT);
     const int split = std::max(1, std::min(chunks, (2 * 152 + blocks - 1) / blocks));
-    k_conv_grad<S, HO><<<dim3(cout / 32, cin / 32, split), 128, G::bytes, st>>>(x, dy, dW, db, n, cin,
-                                                                             cout);
-    return cudaGetLastError();
+    if (split * blocks > kGradCtas) return cudaErrorInvalidValue;
+    float* biasParts = parts + (size_t)kGradCtas * kGradPart;
+    k_conv_grad<S, HO><<<dim3(cout / 32, cin / 32, split), 128, G::bytes, st>>>(x, dy, parts, biasParts,
+                                                                             n, cin, cout);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return sum_grad(parts, biasParts, split, cin, cout, 0, dW, db, st);
 }
 
 }  // namespace
@@ -654,17 +738,25 @@ cudaError_t launch_conv_bwd_data(int layer, const float* dy, const float* wt, co
     }
 }
 
+// the CTAs' parts of a layer's weights, then of its biases
+size_t conv_grad_part_floats() { return (size_t)kGradCtas * (kGradPart + 32); }
+
 cudaError_t launch_conv_bwd_weight(int layer, const float* x, const float* dy, float* dW, float* db,
-                                   int n, int cin, int cout, cudaStream_t st)
+                                   int n, int cin, int cout, float* parts, cudaStream_t st)
 {
     switch (layer) {
-    case 0: k_conv1_grad<<<std::min(n * 32, 152 * 2), 128, 0, st>>>(x, dy, dW, db, n);
-            return cudaGetLastError();
-    case 1: return run_grad<2, 32>(x, dy, dW, db, n, cin, cout, st);
-    case 2: return run_grad<1, 32>(x, dy, dW, db, n, cin, cout, st);
-    case 3: return run_grad<2, 16>(x, dy, dW, db, n, cin, cout, st);
-    case 4: return run_grad<1, 16>(x, dy, dW, db, n, cin, cout, st);
-    case 5: return run_grad<2, 8>(x, dy, dW, db, n, cin, cout, st);
+    case 0: {
+        const int ctas = std::min(n * 32, 152 * 2);
+        float* biasParts = parts + (size_t)kGradCtas * kGradPart;
+        k_conv1_grad<<<ctas, 128, 0, st>>>(x, dy, parts, biasParts, n);
+        const cudaError_t e = cudaGetLastError();
+        return e != cudaSuccess ? e : sum_grad(parts, biasParts, ctas, 1, 32, 1, dW, db, st);
+    }
+    case 1: return run_grad<2, 32>(x, dy, dW, db, n, cin, cout, parts, st);
+    case 2: return run_grad<1, 32>(x, dy, dW, db, n, cin, cout, parts, st);
+    case 3: return run_grad<2, 16>(x, dy, dW, db, n, cin, cout, parts, st);
+    case 4: return run_grad<1, 16>(x, dy, dW, db, n, cin, cout, parts, st);
+    case 5: return run_grad<2, 8>(x, dy, dW, db, n, cin, cout, parts, st);
     default: return cudaErrorInvalidValue;
     }
 }

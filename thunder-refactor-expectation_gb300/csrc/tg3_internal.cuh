@@ -595,6 +595,8 @@ cudaError_t launch_conv_fwd(int layer, const float* x, const float* wt, const fl
                             int n, int cin, int cout, cudaStream_t st);
 cudaError_t launch_conv_bwd_data(int layer, const float* dy, const float* wt, const float* act,
                                  float* dx, int n, int cin, int cout, cudaStream_t st);
+// parts: scratch of conv_grad_part_floats()
+size_t conv_grad_part_floats();
 cudaError_t launch_conv_bwd_weight(int layer, const float* x, const float* dy, float* dW, float* db,
-                                   int n, int cin, int cout, cudaStream_t st);
+                                   int n, int cin, int cout, float* parts, cudaStream_t st);
 }  // namespace tg3
