@@ -1,7 +1,7 @@
 """The network's FP32 convolutions at training batch sizes (the forms that a CTA
-of 32 channels takes, shares of the batch in the weight gradient), and the
-rounding of the weight gradients' long sums, against float64 (torch's
-convolutions on the GPU).
+of 32 channels takes, shares of the batch in the weight gradient), the
+rounding of the weight gradients' long sums, and images with a pixel that is
+not a number, against float64 (torch's convolutions on the GPU).
 
 Weights are -1, 0 and 1, inputs and output gradients whole numbers, so the forward pass and the
 gradients with respect to the activations are exact in FP32 (the largest sums
@@ -119,3 +119,29 @@ def test_sums_keep_their_order():
     for i, (wo, _, bo, co) in enumerate(C.layout()[0]):
         if C.SHAPES[i][4]:
             np.testing.assert_array_equal(a[1][wo:bo + co], b[1][wo:bo + co])
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("n", [3, 40])
+def test_pixels_not_finite(n, value):
+    """A pixel that is not a number: the first layer's outputs over it are 0 by
+    the ReLU and pass no gradient, so all gradients stay finite.  An infinite
+    one with weights of one sign over it does the same where the outputs are
+    -inf."""
+    rng = np.random.default_rng(n)
+    params = _params(rng)
+    if np.isinf(value):
+        w0, ws, _, _ = C.layout()[0][0]
+        params[w0:w0 + int(np.prod(ws))] = -1.0
+    img = rng.integers(-400, 401, (n, 64, 64)).astype(np.float32)
+    img[1, 20, 31] = img[2, 0, 0] = value
+    g_out = rng.integers(-400, 401, (n, tg3.Cnn.N_OUT)).astype(np.float32)
+    bad = torch.as_tensor(~np.isfinite(img)).to(DEV)
+    ref_out, ref, largest = _reference(params, np.nan_to_num(img, nan=0, posinf=0), g_out, bad)
+    assert largest < 2 ** 24
+    out, g = _run(params, img, g_out)
+    assert torch.equal(out.double(), ref_out)
+    for i, (wo, ws, bo, co) in enumerate(C.layout()[0]):
+        if C.SHAPES[i][4]:
+            d, r = np.linalg.norm(g[wo:bo + co] - ref[wo:bo + co]), np.linalg.norm(ref[wo:bo + co])
+            assert d <= 1.7e-7 * r, (i, d / r)

@@ -348,13 +348,20 @@ k_conv_classes(const ConvArgs p)
 // which stays in L2), and the CTAs' parts meet in FP64 in a fixed order
 // (k_grad_sum).  Error of a layer's gradient at 256 images, restated on the CPU:
 // 0.9 to 1.3e-7 of its norm; with one chain a CTA and atomic adds 2.0 to 3.8e-7.
+//
+// A gradient of zero takes no part, whatever it would be multiplied with: the
+// ReLU maps what is not a number to zero and passes no gradient there.  The
+// chains multiply all pairs; a CTA that meets a sum that is not finite does
+// its share again, leaving out the zeros.
 constexpr int kGradChain = 64;                               // a multiple of a chunk's 32
 constexpr int kGradPart = 72 * 128;                          // sums of a CTA
 constexpr int kGradCtas = 320;                               // most CTAs of a launch
 
-// the CTA's sums v[i][k] added to its part (or the first of it)
-__device__ __forceinline__ void add_to_part(uint64_t (&acc)[8][9], float* part, bool first)
+// the CTA's sums v[i][k] added to its part (or the first of it); whether all
+// are finite
+__device__ __forceinline__ bool add_to_part(uint64_t (&acc)[8][9], float* part, bool first)
 {
+    bool finite = true;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         float old[9];
@@ -364,10 +371,12 @@ __device__ __forceinline__ void add_to_part(uint64_t (&acc)[8][9], float* part, 
         for (int k = 0; k < 9; k++) {
             const float2 v = unpack2(acc[i][k]);
             const float s = v.x + v.y + old[k];
+            finite &= fabsf(s) < INFINITY;
             part[(i * 9 + k) * 128] = s;
             acc[i][k] = 0ull;
         }
     }
+    return finite;
 }
 
 template <int S, int HO>
@@ -427,7 +436,7 @@ k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __
     const bool bias = blockIdx.y == 0;
     float* part = parts + ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x * kGradPart +
                   (size_t)blockIdx.x * kGradPart + tid;
-    bool first = true;
+    bool finite = true, first = true;
     if (c0 < c1) stage(c0, 0);
     for (int ch = c0; ch < c1; ch++) {
         const int buf = (ch - c0) & 1;
@@ -485,16 +494,36 @@ k_conv_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __
         __syncthreads();
         sb += sc;
         if ((ch + 1 - c0) % (kGradChain / 32) == 0 || ch + 1 == c1) {
-            add_to_part(acc, part, first);
+            finite &= add_to_part(acc, part, first);
             first = false;
         }
     }
     if (bias && lane < 8) biasParts[(size_t)blockIdx.z * cout + co0 + warp * 8 + lane] = (float)sb;
+    if (!__syncthreads_or(!finite)) return;
+    for (int i = 0; i < 8; i++) {
+        double sum[9] = {};
+        for (int ch = c0; ch < c1; ch++) {
+            const int im = ch / CPI, oy0 = ch % CPI * G::RT;
+            const float* xc = x + ((size_t)im * cin + ci0 + lane) * HI * HI;
+            const float* yc = dy + (((size_t)im * cout + co0 + warp * 8 + i) * HO + oy0) * HO;
+            float a[9] = {};
+            for (int p = 0; p < 64; p++) {
+                const float g = yc[p];
+                if (g == 0.f) continue;
+                for (int k = 0; k < 9; k++) {
+                    const int iy = (oy0 + p / HO) * S + k / 3 - 1, ix = p % HO * S + k % 3 - 1;
+                    if (iy >= 0 && iy < HI && ix >= 0 && ix < HI) a[k] = fmaf(g, xc[iy * HI + ix], a[k]);
+                }
+            }
+            for (int k = 0; k < 9; k++) sum[k] += a[k];
+        }
+        for (int k = 0; k < 9; k++) part[(i * 9 + k) * 128] = (float)sum[k];
+    }
 }
 
 // The first layer's weight gradient (one input channel, 64 x 64): a lane per
 // 4 neighbouring pixels, straight from global memory (each gradient is read
-// once: bound by HBM).  Chains and parts as above; a part has a sum of
+// once: bound by HBM).  Chains, parts and zeros as above; a part has a sum of
 // every lane.
 __global__ void __launch_bounds__(128, 2)
 k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ parts,
@@ -513,7 +542,7 @@ k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* _
     }
     float* part = parts + (size_t)blockIdx.x * kGradPart + threadIdx.x;
     const int total = n * GR, step = gridDim.x * 32;
-    bool first = true;
+    bool finite = true, first = true;
     int done = 0;
     for (int e = blockIdx.x * 32 + lane; e < total; e += step) {
         const int im = e / GR, oy = e % GR / (H / 4), c4 = 4 * (e % (H / 4));
@@ -544,7 +573,7 @@ k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* _
                 }
         }
         if (++done % (kGradChain / 2) == 0 || e + step >= total) {
-            add_to_part(acc, part, first);
+            finite &= add_to_part(acc, part, first);
             first = false;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -557,6 +586,24 @@ k_conv1_grad(const float* __restrict__ x, const float* __restrict__ dy, float* _
     for (int i = 0; i < 8; i++) {
         for (int o = 16; o; o >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
         if (lane == 0) biasParts[(size_t)blockIdx.x * 32 + warp * 8 + i] = (float)sum[i];
+    }
+    if (!__syncthreads_or(!finite)) return;
+    for (int i = 0; i < 8; i++) {
+        double s[9] = {};
+        for (int e = blockIdx.x * 32 + lane; e < total; e += step) {
+            const int im = e / GR, oy = e % GR / (H / 4), c4 = 4 * (e % (H / 4));
+            const float* yp = dy + ((size_t)im * 32 + warp * 8 + i) * (H * H) + oy * H + c4;
+            for (int p = 0; p < 4; p++) {
+                const float g = yp[p];
+                if (g == 0.f) continue;
+                for (int k = 0; k < 9; k++) {
+                    const int iy = oy + k / 3 - 1, ix = c4 + p + k % 3 - 1;
+                    if (iy >= 0 && iy < H && ix >= 0 && ix < H)
+                        s[k] += (double)g * x[(size_t)im * H * H + iy * H + ix];
+                }
+            }
+        }
+        for (int k = 0; k < 9; k++) part[(i * 9 + k) * 128] = (float)s[k];
     }
 }
 
