@@ -114,11 +114,13 @@ struct Total {
     }
 };
 
+constexpr int kBgBand = 5888;        // rows of a table, 46 KB; a multiple of a CTA's 32
+
 __global__ void __launch_bounds__(256)
 k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double* __restrict__ st,
            float* __restrict__ st32, const PrepTables t)
 {
-    extern __shared__ int2 rows[];               // [N rounded up to 4] (left, right) of the circle
+    extern __shared__ int2 rows[];               // a band's (left, right) of the circle
     __shared__ Total part[2][8];
     const size_t l = blockIdx.x;
     if (threadIdx.x < 32)
@@ -144,46 +146,50 @@ k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double
     const int half = N / 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const float pivot = im[0];
-    for (int y = threadIdx.x; y < (N + 3) / 4 * 4; y += blockDim.x) {
-        const int j = y - half, q = bgAbove - j * j;
-        int h = -1;                              // the row inside: |i| <= h
-        if (q >= 0) {
-            h = (int)sqrtf((float)q);
-            while (h * h > q) h--;
-            while ((h + 1) * (h + 1) <= q) h++;
-        }
-        rows[y] = y >= N   ? make_int2(0, 0)
-                  : h < 0 ? make_int2(N, 0)
-                          : make_int2(max(half - h, 0), max(half - h - 1, 0));
-    }
-    __syncthreads();
     Total t1{0.f, 0.f}, t2{0.f, 0.f};
-    for (int y0 = 4 * warp; y0 < N; y0 += 4 * nw) {
-        int left[4], n[4], most = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int2 r = rows[y0 + k];
-            left[k] = r.x;
-            n[k] = r.x + r.y;
-            most = max(most, n[k]);
+    for (int band = 0; band < N; band += kBgBand) {
+        const int end = min((N + 3) / 4 * 4, band + kBgBand);
+        __syncthreads();
+        for (int y = band + threadIdx.x; y < end; y += blockDim.x) {
+            const int j = y - half, q = bgAbove - j * j;
+            int h = -1;                              // the row inside: |i| <= h
+            if (q >= 0) {
+                h = (int)sqrtf((float)q);
+                while (h * h > q) h--;
+                while ((h + 1) * (h + 1) <= q) h++;
+            }
+            rows[y - band] = y >= N   ? make_int2(0, 0)
+                      : h < 0 ? make_int2(N, 0)
+                              : make_int2(max(half - h, 0), max(half - h - 1, 0));
         }
-        for (int e = lane; e < most; e += 64) {
-            float v[8];
+        __syncthreads();
+        for (int y0 = band + 4 * warp; y0 < end; y0 += 4 * nw) {
+            int left[4], n[4], most = 0;
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int f = e + 32 * (k & 1), r = k >> 1;
-                const int x = (y0 + r) * N + (f < left[r] ? f : N - n[r] + f);
-                v[k] = __ldg(im + (f < n[r] ? x : 0));
+            for (int k = 0; k < 4; k++) {
+                const int2 r = rows[y0 - band + k];
+                left[k] = r.x;
+                n[k] = r.x + r.y;
+                most = max(most, n[k]);
             }
-            float a1 = 0.f, a2 = 0.f;
+            for (int e = lane; e < most; e += 64) {
+                float v[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const float d = v[k] - pivot;
-                a1 += d;
-                a2 = fmaf(d, d, a2);
+                for (int k = 0; k < 8; k++) {
+                    const int f = e + 32 * (k & 1), r = k >> 1;
+                    const int x = (y0 + r) * N + (f < left[r] ? f : N - n[r] + f);
+                    v[k] = __ldg(im + (f < n[r] ? x : 0));
+                }
+                float a1 = 0.f, a2 = 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const float d = v[k] - pivot;
+                    a1 += d;
+                    a2 = fmaf(d, d, a2);
+                }
+                t1.add(a1);
+                t2.add(a2);
             }
-            t1.add(a1);
-            t2.add(a2);
         }
     }
     t1.warp_sum();
@@ -890,9 +896,7 @@ extern "C" int tg3_prepare_images_d(tg3_ctx* c, const float* img, int nImg, int 
     const PrepTables tabs{(float*)(b + oM), sm.qIn, nMask, r, ew, (float2*)(b + oT), pl.A, pl.B,
                           (int*)(b + oL), c->px.iCol, c->px.iRow, pl.A ? K : 0, pl.cols, maxCol,
                           pl.W};
-    const size_t rowsB = sizeof(int2) * ((size_t)(N + 3) / 4 * 4);
-    if (rowsB > 47 * 1024)
-        TG3_CUDA(allow_shared(k_bg_stats));
+    const size_t rowsB = sizeof(int2) * (size_t)std::min((N + 3) / 4 * 4, kBgBand);
     k_bg_stats<<<nImg, 256, rowsB, s>>>(img, N, bgAbove, (double)cnt, stv, stats, tabs);
     TG3_LAUNCH_CHECK("background statistics");
     k_stdn<<<1, 256, 0, s>>>(stv, nImg, stdN, sc);
