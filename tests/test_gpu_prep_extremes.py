@@ -1,5 +1,6 @@
 """Image preprocessing of images whose rows exceed one table of the background
-sums (5,888 rows), against float64 sums on the GPU.
+sums (5,888 rows), against float64 sums on the GPU, and of pixels whose
+squares add up to more than FP32 holds, against the float64 oracle.
 
 Tolerances: as in test_gpu_prep_sizes.py, 10 log2(N^2) 2^-24 of the largest
 value; the statistics are FP64 results rounded to FP32."""
@@ -8,6 +9,7 @@ import pytest
 import torch
 
 import tg3
+from oracle import preprocess as PP
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -71,3 +73,19 @@ def test_large_images(N):
         F += ey[:, y:y + rows] @ (v.to(torch.complex128) @ ex)
     ref = F.cpu().numpy()[iRow + 8, iCol]
     assert np.abs(dat[0] - ref).max() <= 10 * np.log2(float(N) ** 2) * 2.0 ** -24 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("N", [48, 64, 94, 256])
+def test_large_pixels(N):
+    """Squares of 1e36, a few thousand to the sum: the statistics and the scaled
+    image are those of the oracle."""
+    rng = np.random.default_rng(N)
+    imgs = (1e18 * rng.standard_normal((3, N, N))).astype(np.float32)
+    imgs[1] *= 1e-18
+    iCol, iRow = _pixels(N // 4)
+    r = 0.3 * N
+    dat, stats = _prepare(torch.as_tensor(imgs).to(DEV), r, iCol, iRow)
+    ref, st, _ = PP.preprocess(imgs, r, iCol, iRow)
+    unit = np.stack([st[:, 1], st[:, 1], np.ones(3)], 1)
+    np.testing.assert_allclose(stats / unit, st / unit, rtol=0, atol=2e-6)
+    assert np.abs(dat - ref).max() <= 10 * np.log2(float(N) ** 2) * 2.0 ** -24 * np.abs(ref).max()

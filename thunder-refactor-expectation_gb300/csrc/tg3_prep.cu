@@ -67,17 +67,7 @@ __device__ __forceinline__ float masked(float v, int q, const SoftMask& k, const
     return q > k.qOut ? 0.f : v * w;
 }
 
-// Per-image background statistics: st[l] = (m, s, sN, 1 / s), sN the background
-// standard deviation of (x - m) / s about 0.  One pass over the background's
-// pixels only, i^2 + j^2 > bgAbove = floor(r^2) in integers: a warp takes four
-// rows at a time, lanes over what lies left and right of the circle, eight
-// loads in flight; a lane sums eight pixels about a pivot (the corner pixel,
-// always background) in FP32 and adds that to totals held as a pair of FP32
-// (the sum and what its roundings lost, 48 bits together), which become FP64 at
-// the end: FP64 sums on the way, two lanes a clock, took most of the time.
-// Lanes past a row's end read the pivot, which adds nothing.  CTA per image;
-// 1,024 images of 256^2: 52 us (a load at a time and FP64 sums: 124).
-// The call's tables come along, spread over the CTAs: the soft mask's edge, w =
+// Tables of a call, spread over the CTAs of k_bg_stats: the soft mask's edge, w =
 // 1 - (0.5 - 0.5 cos((u - r) / ew pi)); the transform's twiddles w_N^(r j)
 // [A][B]; and where the pixels lie in the transform's columns.
 struct PrepTables {
@@ -100,10 +90,8 @@ struct Total {
         lost += (s - (t - b)) + (v - b);
         s = t;
     }
-    __device__ __forceinline__ double value() const
-    {
-        return isinf(s) ? (double)s : (double)s + lost;
-    }
+    __device__ __forceinline__ void add_square(float v) { add(v * v); }
+    __device__ __forceinline__ double value() const { return (double)s + lost; }
     __device__ __forceinline__ void warp_sum()
     {
         for (int o = 16; o; o >>= 1) {
@@ -114,14 +102,128 @@ struct Total {
     }
 };
 
-constexpr int kBgBand = 5888;        // rows of a table, 46 KB; a multiple of a CTA's 32
+// a total in FP64, for sums that leave FP32
+struct WideTotal {
+    double s, none;
+    __device__ __forceinline__ void add(float v) { s += v; }
+    __device__ __forceinline__ void add_square(float v) { s += (double)v * v; }
+    __device__ __forceinline__ double value() const { return s; }
+    __device__ __forceinline__ void warp_sum()
+    {
+        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+};
 
+// The sums of d and d^2 over an image's background pixels only, d = x minus the
+// corner pixel (always background); i^2 + j^2 > bgAbove = floor(r^2) in
+// integers.  A warp takes four rows at a time, lanes over what lies left and
+// right of the circle, eight loads in flight.  A lane sums kTogether pixels in
+// pairs in FP32 and adds that to its totals (T): a pair of FP32 (the sum and what
+// its roundings lost, 48 bits together), which become FP64 at the end: FP64 sums
+// on the way, two lanes a clock, took most of the time.  Lanes past a row's end
+// read the pivot, which adds nothing.  CTA: one image; rows in bands of the
+// table `rows`, (left, right) of the circle.
+//
+// kTogether is 8 from 256 pixels a side and 2 below, where an image has fewer
+// sums for their roundings to cancel over: the deviation of a 64 pixel image is
+// then off by 7.1e-9 (FP32 sums of a row in FP64: 7.0e-9, 8 pixels 8.3e-9), of a
+// 256 pixel one by 4.7e-9 (4.9e-9), root mean squares over images of noise.
+constexpr int kBgBand = 5888;        // 46 KB of rows; a multiple of a CTA's 32
+
+template <int kTogether, class T>
+__device__ __forceinline__ void bg_sums(const float* im, int N, int bgAbove, int2* rows,
+                                        double (&sums)[2])
+{
+    __shared__ T part[2][8];
+    const int half = N / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const float pivot = im[0];
+    T t1{}, t2{};
+    for (int band = 0; band < N; band += kBgBand) {
+        const int end = min((N + 3) / 4 * 4, band + kBgBand);
+        __syncthreads();
+        for (int y = band + threadIdx.x; y < end; y += blockDim.x) {
+            const int j = y - half, q = bgAbove - j * j;
+            int h = -1;                              // the row inside: |i| <= h
+            if (q >= 0) {
+                h = (int)sqrtf((float)q);
+                while (h * h > q) h--;
+                while ((h + 1) * (h + 1) <= q) h++;
+            }
+            rows[y - band] = y >= N   ? make_int2(0, 0)
+                             : h < 0 ? make_int2(N, 0)
+                                     : make_int2(max(half - h, 0), max(half - h - 1, 0));
+        }
+        __syncthreads();
+        for (int y0 = band + 4 * warp; y0 < end; y0 += 4 * nw) {
+            int left[4], n[4], most = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int2 r = rows[y0 - band + k];
+                left[k] = r.x;
+                n[k] = r.x + r.y;
+                most = max(most, n[k]);
+            }
+            for (int e = lane; e < most; e += 64) {
+                float d[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int f = e + 32 * (k & 1), r = k >> 1;
+                    const int x = (y0 + r) * N + (f < left[r] ? f : N - n[r] + f);
+                    d[k] = __ldg(im + (f < n[r] ? x : 0)) - pivot;
+                }
+                if constexpr (kTogether == 1) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        t1.add(d[k]);
+                        t2.add_square(d[k]);
+                    }
+                } else {
+                    float a[4], b[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        a[k] = d[2 * k] + d[2 * k + 1];
+                        b[k] = fmaf(d[2 * k], d[2 * k], d[2 * k + 1] * d[2 * k + 1]);
+                    }
+                    if constexpr (kTogether == 2) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            t1.add(a[k]);
+                            t2.add(b[k]);
+                        }
+                    } else {
+                        t1.add((a[0] + a[1]) + (a[2] + a[3]));
+                        t2.add((b[0] + b[1]) + (b[2] + b[3]));
+                    }
+                }
+            }
+        }
+    }
+    t1.warp_sum();
+    t2.warp_sum();
+    if (lane == 0) {
+        part[0][warp] = t1;
+        part[1][warp] = t2;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double s = 0.0;
+        for (int w = 0; w < nw; w++) s += part[threadIdx.x][w].value();
+        sums[threadIdx.x] = s;
+    }
+    __syncthreads();
+}
+
+// Per-image background statistics: st[l] = (m, s, sN, 1 / s), sN the background
+// standard deviation of (x - m) / s about 0.  Sums that leave FP32 (pixels
+// beyond about 1e17 at 256 a side) are taken again in FP64.  CTA per image; 1,024
+// images of 256^2: 52 us (a load at a time and FP64 sums: 124).
 __global__ void __launch_bounds__(256)
 k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double* __restrict__ st,
            float* __restrict__ st32, const PrepTables t)
 {
-    extern __shared__ int2 rows[];               // a band's (left, right) of the circle
-    __shared__ Total part[2][8];
+    extern __shared__ int2 rows[];               // [N rounded up to 4, kBgBand at most]
+    __shared__ double sums[2];
     const size_t l = blockIdx.x;
     if (threadIdx.x < 32)
         for (int e = blockIdx.x * 32 + threadIdx.x; e < t.A * t.B; e += gridDim.x * 32) {
@@ -143,68 +245,15 @@ k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double
         }
     }
     const float* im = img + l * N * N;
-    const int half = N / 2;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const float pivot = im[0];
-    Total t1{0.f, 0.f}, t2{0.f, 0.f};
-    for (int band = 0; band < N; band += kBgBand) {
-        const int end = min((N + 3) / 4 * 4, band + kBgBand);
-        __syncthreads();
-        for (int y = band + threadIdx.x; y < end; y += blockDim.x) {
-            const int j = y - half, q = bgAbove - j * j;
-            int h = -1;                              // the row inside: |i| <= h
-            if (q >= 0) {
-                h = (int)sqrtf((float)q);
-                while (h * h > q) h--;
-                while ((h + 1) * (h + 1) <= q) h++;
-            }
-            rows[y - band] = y >= N   ? make_int2(0, 0)
-                      : h < 0 ? make_int2(N, 0)
-                              : make_int2(max(half - h, 0), max(half - h - 1, 0));
-        }
-        __syncthreads();
-        for (int y0 = band + 4 * warp; y0 < end; y0 += 4 * nw) {
-            int left[4], n[4], most = 0;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int2 r = rows[y0 - band + k];
-                left[k] = r.x;
-                n[k] = r.x + r.y;
-                most = max(most, n[k]);
-            }
-            for (int e = lane; e < most; e += 64) {
-                float v[8];
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int f = e + 32 * (k & 1), r = k >> 1;
-                    const int x = (y0 + r) * N + (f < left[r] ? f : N - n[r] + f);
-                    v[k] = __ldg(im + (f < n[r] ? x : 0));
-                }
-                float a1 = 0.f, a2 = 0.f;
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const float d = v[k] - pivot;
-                    a1 += d;
-                    a2 = fmaf(d, d, a2);
-                }
-                t1.add(a1);
-                t2.add(a2);
-            }
-        }
-    }
-    t1.warp_sum();
-    t2.warp_sum();
-    if (lane == 0) {
-        part[0][warp] = t1;
-        part[1][warp] = t2;
-    }
-    __syncthreads();
+    if (N < 256)
+        bg_sums<2, Total>(im, N, bgAbove, rows, sums);
+    else
+        bg_sums<8, Total>(im, N, bgAbove, rows, sums);
+    if (!(fabs(sums[0]) < INFINITY && fabs(sums[1]) < INFINITY))
+        bg_sums<1, WideTotal>(im, N, bgAbove, rows, sums);
     if (threadIdx.x == 0) {
-        double s1 = 0.0, s2 = 0.0;
-        for (int w = 0; w < nw; w++) {
-            s1 += part[0][w].value();
-            s2 += part[1][w].value();
-        }
+        const float pivot = im[0];
+        const double s1 = sums[0], s2 = sums[1];
         const double mu = s1 / cnt;                 // mean about the pivot
         const double ss = fmax(s2 - s1 * mu, 0.0);  // sum of (x - m)^2
         const double sd = sqrt(ss / (cnt - 1.0));
