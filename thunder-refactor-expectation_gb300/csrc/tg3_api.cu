@@ -45,6 +45,7 @@ void* ws_get(tg3_ctx* c, WsSlot s, size_t bytes, int* status)
             cudaFree(b.ptr);
             b.ptr = nullptr;
             b.bytes = 0;
+            c->memGen++;
         }
         size_t want = round_up(bytes + bytes / 8, (size_t)2 << 20);
         cudaError_t e = cudaMalloc(&b.ptr, want);
@@ -406,6 +407,7 @@ extern "C" int tg3_ctx_set_volume(tg3_ctx* c, int cls, const float* volume, int 
         cudaFree(v.blocks);
         v.blocks = nullptr;
         v.bytes = 0;
+        c->memGen++;
         TG3_CUDA(cudaMalloc(&v.blocks, bytes));
         v.bytes = bytes;
     }
@@ -454,6 +456,7 @@ static int upload_pixels(tg3_ctx* c, Pixels& px, const int* iCol, const int* iRo
         cudaFree(px.iRow);
         px.iCol = px.iRow = nullptr;
         px.K = 0;
+        c->memGen++;
         TG3_CUDA(cudaMalloc(&px.iCol, sizeof(int) * K));
         TG3_CUDA(cudaMalloc(&px.iRow, sizeof(int) * K));
     }

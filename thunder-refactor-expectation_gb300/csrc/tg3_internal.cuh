@@ -218,6 +218,8 @@ struct tg3_ctx {
     tg3::BankView* d_bankTable = nullptr;    // device copy of the views
     tg3::RefView* d_refTable = nullptr;      // device copy of the reference views
     unsigned pixGen = 0;                     // pixel uploads so far
+    unsigned long long memGen = 0;           // device buffers replaced so far: what was captured
+                                             // with their addresses is captured again
     tg3::Buffer ws[tg3::WS_COUNT];
     int* d_flag = nullptr;           // device error word
     char* pin = nullptr;             // pinned staging of the host-array calls (grow-only), its

@@ -184,6 +184,7 @@ struct tg3_plan {
     RaggedIn in;
     RaggedOut out;
     std::vector<int> clsH, nRH, nTH;
+    int pixels[kMaxClasses] = {};    // of the classes' slots, which size the buffers and offsets
     std::vector<Wave> waves;
     // device: per-particle shapes and offsets, the waves' particle lists
     int* dCls = nullptr;
@@ -197,9 +198,19 @@ struct tg3_plan {
     WaveBuf wb;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    bool replay = false;             // runs replay a graph
+    unsigned long long memGen = 0;   // the context's when it was captured
 };
 
 namespace {
+
+void plan_free_graph(tg3_plan* p)
+{
+    if (p->exec) cudaGraphExecDestroy(p->exec);
+    if (p->graph) cudaGraphDestroy(p->graph);
+    p->exec = nullptr;
+    p->graph = nullptr;
+}
 
 void plan_free_waves(tg3_plan* p)
 {
@@ -207,10 +218,7 @@ void plan_free_waves(tg3_plan* p)
     cudaFree(p->waveMem);
     p->dIdx = nullptr;
     p->waveMem = nullptr;
-    if (p->exec) cudaGraphExecDestroy(p->exec);
-    if (p->graph) cudaGraphDestroy(p->graph);
-    p->exec = nullptr;
-    p->graph = nullptr;
+    plan_free_graph(p);
 }
 
 // Cut the batch into waves for a projection-bank budget and size the wave
@@ -325,6 +333,8 @@ int plan_issue_waves(tg3_plan* p)
     for (const Wave& w : p->waves) {
         if ((st = tg3_ctx_use_pixels(c, w.cls))) return st;
         const int K = c->px.K;
+        if (K != p->pixels[w.cls])
+            return fail(TG3_ERR_STATE, "a class's pixel slot has another size than the plan's");
         k_ragged_gather<<<w.w, 256, 0, s>>>(p->dIdx + w.first, K, w.nR, w.nT, p->dPixOff, p->dROff,
                                              p->dTOff, p->dCls, p->dNR, p->dNT, p->in, p->wb);
         TG3_LAUNCH_CHECK("ragged gather");
@@ -366,6 +376,37 @@ int plan_time(tg3_plan* p, float* ms)
     return tg3_ctx_sync(c);
 }
 
+// The plan's launches as a graph.  It holds the addresses of the context's
+// buffers, so it serves until one of them is replaced (memGen): another call
+// whose workspace is larger, a second plan, a new volume or pixel set.
+int plan_capture(tg3_plan* p)
+{
+    tg3_ctx* c = p->c;
+    plan_free_graph(p);
+    const bool timing = c->timing;
+    c->timing = false;
+    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed);
+    if (e == cudaSuccess) {
+        const int st = plan_issue(p);
+        cudaGraph_t g = nullptr;
+        e = cudaStreamEndCapture(c->stream, &g);
+        if (st || e != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            c->timing = timing;
+            return st ? st : cuda_fail(e, "graph capture");
+        }
+        p->graph = g;
+        e = cudaGraphInstantiate(&p->exec, g, 0);
+    }
+    c->timing = timing;
+    if (e != cudaSuccess) {
+        p->exec = nullptr;
+        return cuda_fail(e, "graph instantiation");
+    }
+    p->memGen = c->memGen;
+    return TG3_OK;
+}
+
 }  // namespace
 
 extern "C" int tg3_ragged_plan_create(
@@ -402,6 +443,7 @@ extern "C" int tg3_ragged_plan_create(
     p->nP = nP;
     p->precision = precision;
     p->clsH.assign(cls, cls + nP);
+    for (int k = 0; k < kMaxClasses; k++) p->pixels[k] = c->pxSlot[k].K;
     p->nRH.assign(nR, nR + nP);
     p->nTH.assign(nT, nT + nP);
     p->in = RaggedIn{reinterpret_cast<const float2*>(dat), ctf, sigRcp, quat, trans, pwR, pwT,
@@ -486,26 +528,9 @@ extern "C" int tg3_ragged_plan_create(
         c->timing = timing;
         return fail_free(st);
     }
-    if (use_graph) {
-        cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed);
-        if (e == cudaSuccess) {
-            st = plan_issue(p);
-            cudaGraph_t g = nullptr;
-            const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
-            if (st || e2 != cudaSuccess) {
-                if (g) cudaGraphDestroy(g);
-                c->timing = timing;
-                return fail_free(st ? st : cuda_fail(e2, "graph capture"));
-            }
-            p->graph = g;
-            e = cudaGraphInstantiate(&p->exec, g, 0);
-        }
-        if (e != cudaSuccess) {
-            c->timing = timing;
-            return fail_free(cuda_fail(e, "graph instantiation"));
-        }
-    }
     c->timing = timing;
+    p->replay = use_graph != 0;
+    if (p->replay && (st = plan_capture(p))) return fail_free(st);
     *out = p;
     return TG3_OK;
 }
@@ -513,7 +538,13 @@ extern "C" int tg3_ragged_plan_create(
 extern "C" int tg3_ragged_plan_run(tg3_plan* p)
 {
     if (!p) return fail(TG3_ERR_ARG, "null plan");
-    if (p->exec) {
+    if (p->replay && (!p->exec || p->memGen != p->c->memGen)) {
+        int st = check_ctx(p->c);
+        if (st) return st;
+        TG3_CUDA(cudaStreamSynchronize(p->c->stream));   // the runs of the graph that goes
+        if ((st = plan_capture(p))) return st;
+    }
+    if (p->replay) {
         TG3_CUDA(cudaGraphLaunch(p->exec, p->c->stream));
         return TG3_OK;
     }
