@@ -297,6 +297,28 @@ extern "C" int tg3_getAviDevice(int* gpus, int cap, int* n)
 }
 
 // ================================================================== context
+// Living contexts of a device that have run a local phase: their launches may
+// meet on the device.  Chooses between forms of the same sums only.
+static std::mutex g_localMutex;
+static int g_localContexts[64];
+static int& local_contexts(const tg3_ctx* c) { return g_localContexts[std::min(c->device, 63)]; }
+
+bool tg3::beside_others(const tg3_ctx* c)
+{
+    std::lock_guard<std::mutex> lock(g_localMutex);
+    return local_contexts(c) > 1;
+}
+
+// c's device must be the current one
+static cudaError_t count_local(tg3_ctx* c, bool enter)
+{
+    if (c->localPhases == enter) return cudaSuccess;
+    std::lock_guard<std::mutex> lock(g_localMutex);
+    c->localPhases = enter;
+    const int n = local_contexts(c) += enter ? 1 : -1;
+    return n == (enter ? 2 : 1) ? prefer_carveouts(enter) : cudaSuccess;
+}
+
 extern "C" int tg3_ctx_create(tg3_ctx** out, int device)
 {
     if (!out) return fail(TG3_ERR_ARG, "null output");
@@ -311,7 +333,6 @@ extern "C" int tg3_ctx_create(tg3_ctx** out, int device)
     if (e == cudaSuccess) e = cudaMemset(c->d_flag, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&c->d_volTable, sizeof(float4*) * kMaxClasses);
     if (e == cudaSuccess) e = cudaMemset(c->d_volTable, 0, sizeof(float4*) * kMaxClasses);
-    if (e == cudaSuccess) e = prefer_carveouts();
     if (e == cudaSuccess) {
         e = cudaMallocHost((void**)&c->pin, kPinFirst);   // enough for a particle's usual call
         if (e == cudaSuccess) c->pinBytes = kPinFirst;
@@ -330,6 +351,7 @@ extern "C" int tg3_ctx_destroy(tg3_ctx* c)
     if (!c) return TG3_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
+    count_local(c, false);
     prep_release(c);
     reco_release(c);
     for (auto& v : c->vol) cudaFree(v.blocks);
@@ -535,6 +557,7 @@ static int local_phase(tg3_ctx* c, const int* bankIdx, int nP, int nR, int nT, c
             return fail(TG3_ERR_ARG, "all class volumes must share one edge and pf");
     if ((st = check_geometry(c, v0.vdim, v0.pf))) return st;
     if ((st = check_weights_shape(nR, nT))) return st;
+    TG3_CUDA(count_local(c, true));
     const bool fusedPath = precision == TG3_SCORE_BF16X3 && c->fused && !bankIdx;
     float* P = fusedPath ? nullptr
                          : (float*)ws_get(c, WS_P, sizeof(float) * (size_t)nP * nR * Kp, &st);
@@ -645,7 +668,8 @@ static int local_phase(tg3_ctx* c, const int* bankIdx, int nP, int nR, int nT, c
         if (split)
             TG3_CUDA(launch_gemm_nt_bf16x3(P, (long long)nR * Kp, Kp, A, (long long)nT * Kp, Kp,
                                            nR, nT, Kp, nP, D, (long long)nR * nT, nT, nrm, nR,
-                                           -2.0f, nullptr, 0, c->d_flag, s, c->localBK));
+                                           -2.0f, nullptr, 0, c->d_flag, s, c->localBK,
+                                           beside_others(c)));
         else
             TG3_CUDA(launch_gemm_nt_fp32(P, (long long)nR * Kp, Kp, A, (long long)nT * Kp, Kp, nR,
                                          nT, Kp, nP, D, (long long)nR * nT, nT, nrm, nR, -2.0f,
@@ -705,6 +729,7 @@ static int local_phase_ctf(tg3_ctx* c, int nP, int nR, int nT, int nD, const flo
     if (!v0.blocks) return fail(TG3_ERR_STATE, "volume of class 0 not set");
     if ((st = check_geometry(c, v0.vdim, v0.pf))) return st;
     if ((st = check_weights_shape(nR, nT))) return st;
+    TG3_CUDA(count_local(c, true));
     const int nTD = nD * nT;
     float* P = (float*)ws_get(c, WS_P, sizeof(float) * (size_t)nP * nR * Kp, &st);
     if (!P) return st;
@@ -754,7 +779,8 @@ static int local_phase_ctf(tg3_ctx* c, int nP, int nR, int nT, int nD, const flo
         if (split)
             TG3_CUDA(launch_gemm_nt_bf16x3(P, (long long)nR * Kp, Kp, A, (long long)nTD * Kp, Kp,
                                            nR, nTD, Kp, nP, D, (long long)nR * nTD, nTD, nullptr,
-                                           nR, -2.0f, nullptr, 0, c->d_flag, s));
+                                           nR, -2.0f, nullptr, 0, c->d_flag, s, 64,
+                                           beside_others(c)));
         else
             TG3_CUDA(launch_gemm_nt_fp32(P, (long long)nR * Kp, Kp, A, (long long)nTD * Kp, Kp,
                                          nR, nTD, Kp, nP, D, (long long)nR * nTD, nTD, nullptr,

@@ -222,6 +222,7 @@ struct tg3_ctx {
                                              // with their addresses is captured again
     tg3::Buffer ws[tg3::WS_COUNT];
     int* d_flag = nullptr;           // device error word
+    bool localPhases = false;        // counted by beside_others
     char* pin = nullptr;             // pinned staging of the host-array calls (grow-only), its
     size_t pinBytes = 0;             // first kPinHead bytes for the error word
     // tg3_ctx_set_option
@@ -529,7 +530,7 @@ cudaError_t launch_gemm_nt_bf16x3(const float* A, long long sA, int lda,
                                   long long sC, int ldc, const float* nrm,
                                   long long sN, float alpha, void* scratch,
                                   size_t scratchBytes, int* flag,
-                                  cudaStream_t st, int bk = 64);
+                                  cudaStream_t st, int bk = 64, bool besideProjections = false);
 size_t bf16x3_scratch_bytes(int M, int N, int Kd, int batch);
 // General split-bf16 GEMM over `items` (see tg3_tc.cu): A/B point at hi
 // planes followed by lo planes of rowsA / rowsB rows of Kd bf16 elements.
@@ -542,7 +543,10 @@ size_t bf16x3_scratch_bytes(int M, int N, int Kd, int batch);
 // split to its end: 3.9 ms at up to 64 KB of shared memory, 4.1 at 132, 4.6 at
 // 164, 7.8 above.  Three contexts' local phases in turn take 5.1 ms each with
 // the GEMM, the shift bank and the resampling kept so (prefer_carveouts), 6.2
-// to 7.0 ms without; alone the GEMM's third stage was worth 0.16 of 5.2 ms.
+// to 7.0 ms without.  A context alone on its device leaves the L1 to nobody: with
+// all of the stages its GEMM takes 1.72 instead of 1.99 of 11.0 ms (128 particles of
+// 1,000 x 100 x 9,930), with the default split its shift bank 0.299 instead of
+// 0.314 (beside_others).
 struct TileBest {
     int* key;
     int rows, groups;
@@ -556,8 +560,11 @@ cudaError_t launch_gemm_bf16x3(const void* A, long long rowsA, const void* B, lo
                                cudaStream_t st, int cGroup = 0, long long cGroupStride = 0,
                                int bk = 64, const TileBest* best = nullptr, bool besideProjections = false);
 // Shared-memory preferences of the kernels that run beside projections, for
-// the current device.
-cudaError_t prefer_carveouts();
+// the current device; with beside 0 the defaults.
+cudaError_t prefer_carveouts(bool beside);
+// Whether the local phases of two or more living contexts have run on c's
+// device.  The same sums either way.
+bool beside_others(const tg3_ctx* c);
 cudaError_t launch_fill_int(int* p, size_t n, int value, cudaStream_t st);
 
 }  // namespace tg3

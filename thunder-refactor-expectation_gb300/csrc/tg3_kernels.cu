@@ -3037,14 +3037,15 @@ cudaError_t launch_nrm_classes(const float* nrm, int nK, int nR, int n, float* o
     return cudaGetLastError();
 }
 
-cudaError_t prefer_carveouts()
+cudaError_t prefer_carveouts(bool beside)
 {
     // half of the SM's memory as L1: their own full occupancy would take up to
     // 200 KB as shared memory (8 CTAs of 25 KB)
+    const int percent = beside ? 50 : cudaSharedmemCarveoutDefault;
     cudaError_t e = cudaFuncSetAttribute(k_shift_bank, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         50);
+                                         percent);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_resample, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
+        e = cudaFuncSetAttribute(k_resample, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
     return e;
 }
 

@@ -200,6 +200,7 @@ struct tg3_plan {
     cudaGraphExec_t exec = nullptr;
     bool replay = false;             // runs replay a graph
     unsigned long long memGen = 0;   // the context's when it was captured
+    bool beside = false;             // and whether others run local phases
 };
 
 namespace {
@@ -378,7 +379,8 @@ int plan_time(tg3_plan* p, float* ms)
 
 // The plan's launches as a graph.  It holds the addresses of the context's
 // buffers, so it serves until one of them is replaced (memGen): another call
-// whose workspace is larger, a second plan, a new volume or pixel set.
+// whose workspace is larger, a second plan, a new volume or pixel set; and the
+// forms that suit a context alone or beside others.
 int plan_capture(tg3_plan* p)
 {
     tg3_ctx* c = p->c;
@@ -404,6 +406,7 @@ int plan_capture(tg3_plan* p)
         return cuda_fail(e, "graph instantiation");
     }
     p->memGen = c->memGen;
+    p->beside = beside_others(c);
     return TG3_OK;
 }
 
@@ -538,7 +541,7 @@ extern "C" int tg3_ragged_plan_create(
 extern "C" int tg3_ragged_plan_run(tg3_plan* p)
 {
     if (!p) return fail(TG3_ERR_ARG, "null plan");
-    if (p->replay && (!p->exec || p->memGen != p->c->memGen)) {
+    if (p->replay && (!p->exec || p->memGen != p->c->memGen || p->beside != beside_others(p->c))) {
         int st = check_ctx(p->c);
         if (st) return st;
         TG3_CUDA(cudaStreamSynchronize(p->c->stream));   // the runs of the graph that goes
