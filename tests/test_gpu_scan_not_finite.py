@@ -103,3 +103,19 @@ def test_minus_infinity(ctx, nImg, nR, nT, precision):
     for got, want in ((wR, e @ i["pT"]), (wT, torch.einsum("lrt,r->lt", e, i["pR"])),
                       (wC, torch.einsum("lrt,r,t->l", e, i["pR"], i["pT"]))):
         torch.testing.assert_close(got, want, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("precision", PRECISIONS, ids=["split", "fp32"])
+@pytest.mark.parametrize("nImg,nR,nT", [(3, 5, 9), (2, 130, 33), (5, 64, 49), (2, 70, 200)])
+def test_infinite_prior(ctx, nImg, nR, nT, precision):
+    """An infinite prior of one translation and log-likelihoods within a few units
+    of one another: every rotation's weight and the image's are infinite, the
+    translations' finite."""
+    i = _inputs(ctx, nImg, nR, nT)
+    i["sig"] *= 1e-5
+    i["pT"][nT // 2] = float("inf")
+    wC, wR, wT, base, L = _scan(ctx, i, nImg, nR, nT, precision)
+    assert float((base[:, None, None] - L).max()) < 60
+    assert (wR == float("inf")).all() and (wC == float("inf")).all()
+    torch.testing.assert_close(wT, torch.einsum("lrt,r->lt", torch.exp(L - base[:, None, None]),
+                                                i["pR"]), rtol=1e-4, atol=0)

@@ -1577,6 +1577,8 @@ k_weights(const float* __restrict__ D, long long sD, int ldc, int nR, int nT, in
             float sr = (b3 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b3 ? s0 : s1, 8);
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, o);
+            // a row past the end has a prior of 0, but its sum may be infinite
+            if (!whole && r0 + (lane >> 3) * nw >= nR) sr = 0.f;
 #pragma unroll
             for (int q = 0; q < 4; q++)      // sum_t s pT[t] pR[r], once per row
                 cacc = fmaf(__shfl_sync(0xffffffffu, sr, 8 * q), prr[q], cacc);
