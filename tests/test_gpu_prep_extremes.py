@@ -89,3 +89,38 @@ def test_large_pixels(N):
     unit = np.stack([st[:, 1], st[:, 1], np.ones(3)], 1)
     np.testing.assert_allclose(stats / unit, st / unit, rtol=0, atol=2e-6)
     assert np.abs(dat - ref).max() <= 10 * np.log2(float(N) ** 2) * 2.0 ** -24 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("N", [64, 94, 256])
+def test_pixels_not_finite(N):
+    """A NaN background pixel, an infinite one, a NaN corner (the sums' pivot) and a
+    NaN inside the circle: such an image's mean or deviation is not a finite number
+    (the last one's are, only its pixel data is not), the other images' results are
+    the same bits as without them."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    img = torch.randn((6, N, N), generator=g, device=DEV) * 3 + 2
+    iCol, iRow = _pixels(N // 4)
+    r = 0.4 * N
+
+    def run(x):
+        ctx = tg3.Context(0)
+        try:
+            ctx.set_pixels(iCol, iRow, N)
+            dat = torch.empty((6, len(iCol)), dtype=torch.complex64, device=DEV)
+            stats = torch.empty((6, 3), dtype=torch.float32, device=DEV)
+            torch.cuda.synchronize()
+            ctx.prepare_images(x, r, dat, std_n=1.0, stats=stats)
+            ctx.sync()
+        finally:
+            ctx.close()
+        return dat, stats
+
+    dat, stats = run(img)
+    bad = img.clone()
+    bad[0, 1, N // 2] = bad[2, 0, 0] = bad[3, N // 2, N // 2] = float("nan")
+    bad[1, N - 1, 3] = float("inf")
+    dat2, stats2 = run(bad)
+    for k in (4, 5):
+        assert torch.equal(dat[k], dat2[k]) and torch.equal(stats[k], stats2[k])
+    assert not stats2[:3].isfinite().all(1).any()
+    assert torch.equal(stats[3], stats2[3]) and dat2[:4].isnan().all()

@@ -170,8 +170,10 @@ __device__ __forceinline__ void bg_sums(const float* im, int N, int bgAbove, int
                 for (int k = 0; k < 8; k++) {
                     const int f = e + 32 * (k & 1), r = k >> 1;
                     const int x = (y0 + r) * N + (f < left[r] ? f : N - n[r] + f);
-                    d[k] = __ldg(im + (f < n[r] ? x : 0)) - pivot;
+                    d[k] = __ldg(im + (f < n[r] ? x : 0));
                 }
+#pragma unroll
+                for (int k = 0; k < 8; k++) d[k] -= pivot;
                 if constexpr (kTogether == 1) {
 #pragma unroll
                     for (int k = 0; k < 8; k++) {
@@ -214,10 +216,18 @@ __device__ __forceinline__ void bg_sums(const float* im, int N, int bgAbove, int
     __syncthreads();
 }
 
+// apart, so that it takes no registers from the usual sums
+__device__ __noinline__ void bg_sums_wide(const float* im, int N, int bgAbove, int2* rows,
+                                          double (&sums)[2])
+{
+    bg_sums<1, WideTotal>(im, N, bgAbove, rows, sums);
+}
+
 // Per-image background statistics: st[l] = (m, s, sN, 1 / s), sN the background
 // standard deviation of (x - m) / s about 0.  Sums that leave FP32 (pixels
 // beyond about 1e17 at 256 a side) are taken again in FP64.  CTA per image; 1,024
-// images of 256^2: 52 us (a load at a time and FP64 sums: 124).
+// images of 256^2: 50 us (a load at a time and FP64 sums: 124).
+template <int kTogether>
 __global__ void __launch_bounds__(256)
 k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double* __restrict__ st,
            float* __restrict__ st32, const PrepTables t)
@@ -245,12 +255,9 @@ k_bg_stats(const float* __restrict__ img, int N, int bgAbove, double cnt, double
         }
     }
     const float* im = img + l * N * N;
-    if (N < 256)
-        bg_sums<2, Total>(im, N, bgAbove, rows, sums);
-    else
-        bg_sums<8, Total>(im, N, bgAbove, rows, sums);
+    bg_sums<kTogether, Total>(im, N, bgAbove, rows, sums);
     if (!(fabs(sums[0]) < INFINITY && fabs(sums[1]) < INFINITY))
-        bg_sums<1, WideTotal>(im, N, bgAbove, rows, sums);
+        bg_sums_wide(im, N, bgAbove, rows, sums);
     if (threadIdx.x == 0) {
         const float pivot = im[0];
         const double s1 = sums[0], s2 = sums[1];
@@ -946,7 +953,8 @@ extern "C" int tg3_prepare_images_d(tg3_ctx* c, const float* img, int nImg, int 
                           (int*)(b + oL), c->px.iCol, c->px.iRow, pl.A ? K : 0, pl.cols, maxCol,
                           pl.W};
     const size_t rowsB = sizeof(int2) * (size_t)std::min((N + 3) / 4 * 4, kBgBand);
-    k_bg_stats<<<nImg, 256, rowsB, s>>>(img, N, bgAbove, (double)cnt, stv, stats, tabs);
+    (N < 256 ? k_bg_stats<2> : k_bg_stats<8>)<<<nImg, 256, rowsB, s>>>(img, N, bgAbove, (double)cnt,
+                                                                      stv, stats, tabs);
     TG3_LAUNCH_CHECK("background statistics");
     k_stdn<<<1, 256, 0, s>>>(stv, nImg, stdN, sc);
     TG3_LAUNCH_CHECK("noise level");
