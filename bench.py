@@ -51,6 +51,9 @@ def peaks():
     return 6800.0, 1900.0, "fallback"
 
 
+SMS = 152                       # of a GB300
+
+
 # ---------------------------------------------------------------- clocks ----
 class ClockSampler:
     """nvidia-smi clock/throttle samples during the timed region."""
@@ -365,13 +368,18 @@ def run_tg3(args, rank, world, local_rank):
                 "executed_bf16_flop_per_launch": 3 * flop if p_ != tg3.SCORE_FP32 else None}
 
     def proj_roof(st_):
-        ach = proj_bytes / (per_launch(st_, "project") * 1e-3) / 1e9
-        return {"kernel": "k_project", "bound": "hbm", "achieved": round(ach, 1),
-                "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4),
-                "peak_source": f"hbm_gbs, {kind} (MEASURED_PEAKS.json)",
-                "traffic": traffic("project", W["box"], nP),
-                "traffic_note": "DRAM bytes per launch (ncu); below the algorithmic bytes "
-                                "because L2 serves the volume blocks a pixel band reuses",
+        # a sample is one 64-byte block, a wavefront of the L1's data stage, which takes one a
+        # clock and SM; L2 serves the blocks that a pixel band reuses, so the algorithmic bytes
+        # are no measure against HBM
+        t = per_launch(st_, "project") * 1e-3
+        ach = nR * K * nP / t / 1e9
+        pk = SMS * (clocks["sm_mhz"] or 2070.0) * 1e-3
+        dram = traffic("project", W["box"], nP)
+        return {"kernel": "k_project_xchg", "bound": "l1", "achieved": round(ach, 1),
+                "peak": round(pk, 1), "unit": "G blocks/s", "frac": round(ach / pk, 4),
+                "peak_source": "one L1 wavefront a clock and SM at the sampled SM clock",
+                "traffic": dram, "traffic_note": "DRAM bytes per launch (ncu)",
+                "traffic_frac_of_hbm": None if dram is None else round(dram / t / 1e9 / hbm, 4),
                 "algorithmic_bytes_per_launch": proj_bytes}
 
     def fused_roof(st_):
@@ -431,7 +439,7 @@ def run_tg3(args, rank, world, local_rank):
         "roofline_projection": None if fused else proj_roof(stages),
         "stages": {k: {"ms_per_launch": round(v[0] / max(v[1], 1), 4), "launches": v[1]}
                    for k, v in stages.items() if v[1]},
-        "insertion": {"kernel": "k_insert (MKB, a = 1.9, alpha = 15)",
+        "insertion": {"kernel": "k_insert_mkb (a = 1.9, alpha = 15)",
                       "particles": nP,
                       "ms_per_launch": round(ins_ms, 4),
                       "particles_per_s": round(nP / (ins_ms * 1e-3), 1),
@@ -839,6 +847,11 @@ def run_prep(args, rank, world, local_rank):
 BANK_KERNELS = {0: "k_gemm_bank_cp (bank rows gathered by cp.async)",
                 1: "k_gemm_bf16x3 (rows copied out of the banks first)",
                 2: "k_gemm_bank_bf16x3 (bank rows gathered by TMA)"}
+# what bounds it: the cp.async form waits for shared memory (copies, norm reads, the tensor
+# cores' operands) and its warps' instructions; the others stream planes from HBM
+BANK_BOUND = {0: "smem", 1: "hbm", 2: "hbm"}
+BANK_FRAC_NOTE = ("algorithmic bytes (each proposed row once) against the HBM rate, for scale: "
+                  "about half of the rows come from L2")
 
 
 def run_bank(args, rank, world, local_rank):
@@ -937,7 +950,8 @@ def run_bank(args, rank, world, local_rank):
                                   f"box-{box} class, bank of {len(qg)} rotations, K = {K}",
                       "l2": "inputs larger than L2 (bank 0.55 GB)"},
            "clocks": clocks,
-           "roofline": {"kernel": BANK_KERNELS[main[0]], "bound": "hbm",
+           "roofline": {"kernel": BANK_KERNELS[main[0]], "bound": BANK_BOUND[main[0]],
+                        "frac_note": BANK_FRAC_NOTE,
                         "achieved": round(ach, 1),
                         "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4),
                         "peak_source": f"hbm_gbs, {kind} (MEASURED_PEAKS.json)",
@@ -1101,13 +1115,19 @@ def run_reco(args, rank, world, local_rank):
     clocks = clk.stop()
     ms = reduce_max(world, e0.elapsed_time(e1)) / steps
     nh = vdim * vdim * (vdim // 2 + 1)
-    nr = vdim ** 3
-    # algorithmic bytes of one balancing round: T, W read and C written
-    # (C = T W), C read and the real map written (inverse), the map read and
-    # written (kernel product), read and C written (forward), C read and W
-    # read and written (update) -- each array once per pass
-    per_round = 4 * nh * 2 + 8 * nh + 8 * nh + 4 * nr + 8 * nr + 4 * nr + 8 * nh + 8 * nh + 8 * nh
-    alg = rounds * per_round + 16 * nh + 8 * nh + 4 * nr + 4 * N ** 3
+    # what the passes move: C has the columns x < rmax in groups of 8, the z pass and one side
+    # of the y passes the lines inside the sphere only; W is read and written and T read
+    # inside it, the kernel's grid over an octant once a round
+    rmax = maxR * pf
+    cols = -(-rmax // 8) * 8
+    lines = sum(8 * (2 * math.isqrt(rmax * rmax - 1 - x * x) + 1) for x in range(0, cols, 8))
+    inside = 2 * math.pi / 3 * rmax ** 3
+    z_pass, y_pass = 8 * 2 * lines * vdim, 8 * (lines + cols * vdim) * vdim
+    per_round = (z_pass + 12 * inside + 2 * y_pass + 8 * 2 * cols * vdim ** 2
+                 + 4 * (vdim // 2 + 1) ** 3)
+    # the sums in; T, W and C set up; F W, half of the planes back, the map out
+    alg = rounds * per_round + 24 * nh + (16 + 8) * inside + z_pass / 2 \
+        + (16 + 4) * inside + z_pass / 2 + (y_pass + 8 * cols * vdim ** 2) / 2 + 4 * N ** 3
     hbm, bf16, kind = peaks()
     achieved = alg / (ms * 1e-3) / 1e9
     ctx.close()
@@ -1117,7 +1137,7 @@ def run_reco(args, rank, world, local_rank):
             "higher_is_better": True, "dtype": "f32",
             "data": "synthetic: padded transform of a 200-blob map, radial T",
             "config": {"workload": "reco256", "box": N, "pf": pf, "max_radius": maxR,
-                       "balancing_rounds": rounds, "l2": "arrays (2.7 GB) larger than L2"},
+                       "balancing_rounds": rounds, "l2": "arrays (2.1 GB) larger than L2"},
             "clocks": clocks,
             "roofline": {"bound": "hbm", "kernel": "whole reconstruction",
                          "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
@@ -1843,8 +1863,8 @@ def learned_rooflines(st, steps, n, nRot, nTrans, K, Kp, nfb, nRg, nTg, bank_for
       rows (4 Kp) out;
     - rescoring cross term (every form): per launch the proposed rows' planes
       (4 Kp bytes a row), the shifted data (4 Kp a translation) and the
-      log-likelihoods (4 bytes a hypothesis): HBM-bound (4 K FLOP per
-      hypothesis, 3x that in bf16, is far below the tensor cores' rate);
+      log-likelihoods (4 bytes a hypothesis); 4 K FLOP per
+      hypothesis, 3x that in bf16, is far below the tensor cores' rate;
     - fallback cross term (the global search of the fallback particles):
       4 K FLOP per hypothesis, nRg x nTg per fallback particle."""
     hbm, bf16, src = peaks()
@@ -1858,12 +1878,13 @@ def learned_rooflines(st, steps, n, nRot, nTrans, K, Kp, nfb, nRg, nTg, bank_for
             "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4),
             "traffic": None, "algorithmic_bytes_per_launch": algo / steps}
     if tot("cross") > 0:
-        # every form streams the proposed rows' planes: HBM-bound
+        # every form streams the proposed rows' planes
         algo = (float(n) * nRot * 4.0 * Kp + float(n) * nTrans * 4.0 * Kp
                 + float(n) * nRot * nTrans * 4.0) * steps
         ach = algo / (tot("cross") * 1e-3) / 1e9
         out["rescoring_cross"] = {
-            "kernel": BANK_KERNELS[bank_form], "bound": "hbm", "achieved": round(ach, 1),
+            "kernel": BANK_KERNELS[bank_form], "bound": BANK_BOUND[bank_form],
+            "frac_note": BANK_FRAC_NOTE, "achieved": round(ach, 1),
             "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4), "traffic": None,
             "algorithmic_bytes_per_launch": algo / steps,
             "tflops_algorithmic": round(4.0 * K * n * nRot * nTrans * steps
@@ -1882,7 +1903,7 @@ def learned_rooflines(st, steps, n, nRot, nTrans, K, Kp, nfb, nRg, nTg, bank_for
                  "fallback_cross": "fallback_cross"}[k]
         v["ms_per_step"] = round(tot(stage) / steps, 4)
         v["share_of_step"] = round(tot(stage) / steps / step_ms, 4)
-        v["peak_source"] = f"{'hbm_gbs' if v['bound'] == 'hbm' else 'bf16_tflops'}, {src} " \
+        v["peak_source"] = f"{'hbm_gbs' if v['unit'] == 'GB/s' else 'bf16_tflops'}, {src} " \
                            "(MEASURED_PEAKS.json)"
     dom = max(out, key=lambda k: out[k]["ms_per_step"]) if out else None
     return dom, out
