@@ -271,8 +271,11 @@ __global__ void k_acc_load(const float2* __restrict__ F, const float* __restrict
 // C is zero and not looked at outside the sphere |k|^2 < r2max, so C keeps the
 // columns x < rmax only, the y passes read (inverse) or write (forward) the
 // rows inside the circle of their column, and the z pass visits those lines
-// only.  Bound by HBM: a round moves about 4 GB at 512^3 with rmax 240 and
-// takes 1.2 ms, where the library's six transform kernels and two passes
+// only.  Bound by the latency of loads, exchanges and stores at 12 warps an SM (DRAM
+// at a quarter to a half of its rate): a thread holds 24 to 32 points at up to 168
+// registers, and 12 of the 17 z passes spill some of them (8 to 216 bytes; 12 at
+// 32 x 16, whose y pass spills 80).  A round moves about 3.9 GB at 512^3 with rmax
+// 240 and takes 1.2 ms, where the library's six transform kernels and two passes
 // between them took 2.35 ms.
 struct Pass3 {
     const float2* tw;        // the n-th roots of unity
